@@ -92,7 +92,8 @@ typedef struct b200fft_launch_record {
   int kind;          /* 0 c2c, 1 r2c, 2 c2r, 3 copy                         */
   int direction;     /* B200FFT_FORWARD / B200FFT_BACKWARD                   */
   int stage;         /* stage index for c2c, -1 otherwise                    */
-  int family;        /* 0 static specialised kernel, 1 runtime generic,
+  int family;        /* 0 static specialised kernel, 1 other lengths (a compiled
+                        mixed-length plan or the runtime-generic kernel),
                         2/3 split-precision tensor core (mma.sync / tcgen05),
                         4 TMA-fed specialised column kernel, -1 copy */
   int length;        /* transform length (real length for r2c/c2r)          */

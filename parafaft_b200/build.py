@@ -40,7 +40,25 @@ NVCC_FLAGS = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC"] + ARCH
 ENGINE_SOURCES = ["api.cu", "fg.cu", "fs_c2c_f32.cu", "fs_c2c_f64.cu",
                   "fs_r2c_f32.cu", "fs_r2c_f64.cu", "fft_tc.cu", "fft_tc5.cu", "fft_tma.cu",
                   "noalloc.cu", "fft_sched.cu", "fs_colpair.cu",
-                  "fft_tc5col.cu"]
+                  "fft_tc5col.cu", "fm.cu"]
+
+# fm_inst.cu is compiled once per precision, form (columns, rows, real rows) and
+# range of lengths; the ranges meet at kMixedCut of fm.cu.
+MIXED_RANGES = [(3, 136), (136, 351), (351, 801), (801, 2049)]
+
+
+def engine_units() -> list[tuple[str, str, list[str]]]:
+    """(source, object name, extra flags) of every engine compilation unit,
+    the longest-running ones first."""
+    units = []
+    for form in (2, 0, 1):
+        for prec in (64, 32):
+            for k, (lo, hi) in reversed(list(enumerate(MIXED_RANGES))):
+                name = f"fm_{prec}_{form}_{k}"
+                units.append(("fm_inst.cu", name, [f"-DFM_PREC={prec}", f"-DFM_FORM={form}",
+                                                   f"-DFM_LO={lo}", f"-DFM_HI={hi}",
+                                                   f"-DFM_NAME={name}"]))
+    return [(s, Path(s).stem, []) for s in ENGINE_SOURCES] + units
 
 
 def _nvcc() -> str:
@@ -78,12 +96,15 @@ def build_engine(force: bool = False) -> Path:
     headers = list(CSRC.glob("*.hpp")) + list(CSRC.glob("*.cuh")) + [INCLUDE / "b200fft.h"]
     jobs = []
     objs = []
-    for src in ENGINE_SOURCES:
+    for src, name, extra in engine_units():
         s = CSRC / src
-        o = OBJ / (s.stem + ".o")
+        o = OBJ / (name + ".o")
         objs.append(o)
         if force or _newer(o, [s] + headers):
-            jobs.append([_nvcc(), *NVCC_FLAGS, "-I", str(INCLUDE), "-c", str(s), "-o", str(o)])
+            # line tables would triple the size of the many mixed-length kernels
+            flags = [f for f in NVCC_FLAGS if not (extra and f == "-lineinfo")]
+            jobs.append([_nvcc(), *flags, *extra, "-I", str(INCLUDE), "-c", str(s),
+                         "-o", str(o)])
     if jobs:
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
             list(ex.map(_run, jobs))

@@ -34,6 +34,7 @@
 #include "../../include/b200fft.h"
 #include "fft_common.hpp"
 #include "launch.hpp"
+#include "mixed_plan.hpp"
 
 using namespace b200fft;
 
@@ -74,6 +75,13 @@ struct Choice {
   int esize = 8;   // bytes per complex element
   int variant = 0; // tile-shape candidate of a specialised kernel
   GenArgs gen{};
+  // the compiled kernel of a length with odd prime factors (fft_mixed.cuh);
+  // nulls in family 1: the runtime-generic kernel
+  MixedKernel mixed;
+
+  // Whether the R2C/C2R kernel takes both sides in complex units (rows of even
+  // real length on the compiled kernels) rather than the real side in reals.
+  bool complex_units() const { return family == 0 || (mixed.one != nullptr && !gen.odd); }
 };
 
 struct Plan {
@@ -166,11 +174,8 @@ int ilog2(int x) {
 // 512 or more points use the 512-thread full tile; everything else the full
 // tile (measured on the 512^3 and 1024^3 passes).
 int default_variant(int csize, int L, bool col, long long stride) {
-  if (col && !is_pow2(L))
-    // FP32 mixed-length columns of up to 256 points: the half tile (still >= 16
-    // transforms; 60/80/120/160 points 6-12% faster as single plans; grouped
-    // launches keep the full tile, where the half tile was slower)
-    return (csize == 8 && L <= 256) ? 1 : 0;
+  if (!is_pow2(L))
+    return 0; // no tile variants: the compiled plan of the length (mixed_plan.hpp)
   if (col) {
     // 2048+ points: the wide tile at any stride (its 2-8 transforms per tile
     // still give 32-64-byte row segments, the full tile's half that: FP32 and
@@ -260,8 +265,13 @@ int choose_kernel(int prec, int kind, int len, long long batch, long long stride
     }
     if (variant >= 0 && variant < kStaticVariants)
       var = variant;
-    if (!is_pow2(L) && !(ch.col && var == 1))
-      var = 0; // mixed-radix lengths: the full tile, or the half tile for columns
+    if (!is_pow2(L)) {
+      // the compiled plans replaced the power-of-two thread mapping of these
+      // lengths: rows and columns of 24..768 points 3.4-6.1 -> 3.9-6.4 TB/s, R2C and
+      // C2R rows 2.1-4.2 -> 3.6-5.8; only the group schedule kernel still runs it
+      var = 0;
+      ch.mixed = mixed_kernel(prec == B200FFT_F64, kind, odd, ch.col, L);
+    }
     if (var == kVariantPair &&
         !(ch.col && kind == KIND_C2C && csize == 8 && colpair_length_ok(L)))
       var = default_variant(csize, L, ch.col, stride); // the pair tile does not apply
@@ -314,6 +324,12 @@ int choose_kernel(int prec, int kind, int len, long long batch, long long stride
   ch.family = 1;
   ch.TB = TB;
   ch.NT = kGenThreads;
+  // Lengths of factors 2, 3, 5, 7 (and one 11 or 13) up to 2048 have a compiled
+  // plan: 4-6.5 TB/s against 0.7-2.8 for the runtime schedule (36 to 1225
+  // points, both layouts and precisions). R2C/C2R rows as for the specialised
+  // kernels: contiguous, an even distance.
+  if (!force_generic && (kind == KIND_C2C || (stride == 1 && dist % 2 == 0)))
+    ch.mixed = mixed_kernel(prec == B200FFT_F64, kind, odd, ch.col, L);
   *out = ch;
   return B200FFT_SUCCESS;
 }
@@ -336,15 +352,23 @@ std::string describe_choice(const Choice &ch, int kind) {
   }
   if (rad.empty())
     rad = "1";
+  std::string compiled; // the plan of the compiled kernel that runs
+  if (ch.mixed.one != nullptr) {
+    const MixedPlan mp = mixed_plan(ch.L, ch.esize, ch.col);
+    for (int s = 0; s < mp.nst; ++s)
+      compiled += (s ? "x" : " compiled=") + std::to_string(mp.rad[s]);
+    compiled += " on " + std::to_string(mp.P) + "x" + std::to_string(mp.TB) + " threads";
+  }
   const char *kn = kind == KIND_C2C ? "c2c" : (kind == KIND_R2C ? "r2c" : "c2r");
-  std::snprintf(buf, sizeof(buf), "%s %s L=%d %s tb=%d nt=%d radices=%s var=%d",
+  std::snprintf(buf, sizeof(buf), "%s %s L=%d %s tb=%d nt=%d radices=%s var=%d%s",
                 ch.family == 0   ? "static"
                 : ch.family == 2 ? "split-tc"
                 : ch.family == 3 ? "split-tc5"
                 : ch.family == 5 ? "split-tc5col"
                                  : "generic",
                 kn, ch.L,
-                ch.col ? "col" : "row", ch.TB, ch.NT, rad.c_str(), ch.variant);
+                ch.col ? "col" : "row", ch.TB, ch.NT, rad.c_str(), ch.variant,
+                compiled.c_str());
   return buf;
 }
 
@@ -416,6 +440,7 @@ struct GroupStep {
   bool f64 = false, col = false, fwd = true;
   int kind = KIND_C2C;
   int L = 0;
+  MixedKernel mixed; // STATIC: the compiled kernel of a mixed length, if it is one
   std::vector<GenArgs> items;
   std::vector<PassArgs> sitems;
   std::vector<long long> tile_start;
@@ -713,9 +738,9 @@ int finish_fused_copy(H *h, const char *out0, size_t covered) {
 // slabs/slab (complex elements) describe a coalesced middle-axis run.
 cudaError_t launch_kernel(H *h, const Plan &p, int dir, const PassArgs &a);
 
-// Kernel arguments of one pass of plan p run by kernel family `family`
-// (element units differ between the specialised and generic R2C/C2R kernels).
-PassArgs pass_args(const Plan &p, int family, const void *in, void *out, const void *tw,
+// Kernel arguments of one pass of plan p; `cunits`: R2C/C2R rows in complex
+// units on both sides (Choice::complex_units).
+PassArgs pass_args(const Plan &p, bool cunits, const void *in, void *out, const void *tw,
                    long long slabs, long long slab) {
   PassArgs a{};
   a.in = in;
@@ -727,7 +752,7 @@ PassArgs pass_args(const Plan &p, int family, const void *in, void *out, const v
     a.idist = a.odist = p.dist;
     a.istride = a.ostride = p.stride;
     a.islab = a.oslab = slab;
-  } else if (family == 0) { // both sides complex units, contiguous rows
+  } else if (cunits) { // both sides complex units, contiguous rows
     a.idist = a.odist = p.dist / 2;
     a.istride = a.ostride = 1;
     a.islab = a.oslab = 0;
@@ -758,7 +783,7 @@ int launch_pass(H *h, const Plan &p, int dir, const void *in, void *out,
                 long long slabs, long long slab, bool fused, int stage, long long in_dist = -1) {
   const void *tw = nullptr;
   B2_TRY(get_table(h, p.ch.tlen, &tw));
-  PassArgs a = pass_args(p, p.ch.family, in, out, tw, slabs, slab);
+  PassArgs a = pass_args(p, p.ch.complex_units(), in, out, tw, slabs, slab);
   if (in_dist >= 0)
     a.idist = in_dist;
   const long long bytes = pass_bytes(h, p, a.total);
@@ -845,7 +870,9 @@ cudaError_t launch_kernel(H *h, const Plan &p, int dir, const PassArgs &a) {
   const bool f64 = h->prec == B200FFT_F64;
   const bool fwd = dir == B200FFT_FORWARD;
   cudaError_t e;
-  if (p.ch.family == 0) {
+  if (p.ch.mixed.one != nullptr) {
+    e = p.ch.mixed.one(a, fwd ? 0u : 0x80000000u, h->stream);
+  } else if (p.ch.family == 0) {
     if (p.kind == KIND_C2C) {
       int var = column_tile_for(h, p, a.total);
       // FP32 512-point columns whose neighbouring transforms sit side by side
@@ -990,7 +1017,7 @@ int time_candidate(H *h, const Plan &q, long long lead, double *ms) {
   const void *tw = nullptr;
   B2_TRY(get_table(h, q.ch.tlen, &tw));
   const long long slab = lead > 1 ? static_cast<long long>(q.len) * q.batch : 0;
-  const PassArgs a = pass_args(q, q.ch.family, h->work, h->work, tw, lead, slab);
+  const PassArgs a = pass_args(q, q.ch.complex_units(), h->work, h->work, tw, lead, slab);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -1025,13 +1052,16 @@ int autotune(H *h, Plan &p) {
   const int rigor = h->plan_flag; // 1 Measure, 2 Patient
   const long long lead = infer_lead(h, p);
   const std::string key = wisdom_key(h, p, lead);
+  // family 1 of an entry or a candidate: the runtime-generic kernel where the
+  // length also has a specialised one, else the plan's own choice
+  const bool has_static = p.ch.family == 0;
   {
     std::lock_guard<std::mutex> lk(g_wis_mu);
     auto it = g_wisdom.find(key);
     if (it != g_wisdom.end() && it->second.rigor >= rigor) {
       Choice c;
       if (choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist,
-                        it->second.family == 1, &c, it->second.variant) == B200FFT_SUCCESS) {
+                        it->second.family == 1 && has_static, &c, it->second.variant) == B200FFT_SUCCESS) {
         p.ch = c;
         return B200FFT_SUCCESS;
       }
@@ -1064,8 +1094,8 @@ int autotune(H *h, Plan &p) {
   WisdomVal wv;
   for (auto fv : cands) {
     Choice c;
-    if (choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, fv.first == 1, &c,
-                      fv.second) != B200FFT_SUCCESS)
+    if (choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist,
+                      fv.first == 1 && has_static, &c, fv.second) != B200FFT_SUCCESS)
       continue;
     if (c.family != fv.first)
       continue;
@@ -1142,7 +1172,7 @@ int exec_real(H *h, Plan &p, int kind, void *ptr) {
     // padded row is overwritten whole, pad lanes included).
     const HeldCopy2D c = h->pad;
     const size_t rs = static_cast<size_t>(h->rsize);
-    const size_t unit = p.ch.family == 0 ? 2 * rs : rs; // input units of the kernel
+    const size_t unit = p.ch.complex_units() ? 2 * rs : rs; // input units of the kernel
     const char *src_end = c.src + c.spitch * (c.height - 1) + c.width;
     const char *dst_end = c.dst + c.dpitch * c.height;
     const bool match = kind == KIND_R2C && c.dst == ptr && p.stride == 1 &&
@@ -1851,7 +1881,7 @@ bool sched_build(G *g, int *rc) {
       if (spec < 0)
         return false;
       SchedPass q{};
-      q.a = pass_args(p, 0, op.in, op.out, op.tw, op.slabs, op.slab);
+      q.a = pass_args(p, true, op.in, op.out, op.tw, op.slabs, op.slab);
       q.spec = spec;
       const long long tb = sched_tile_transforms(spec);
       const long long nt = (q.a.total + tb - 1) / tb;
@@ -1989,13 +2019,37 @@ int group_build(G *g) {
       // A pass with a specialised kernel joins the grouped launch of that
       // kernel (same length, layout, kind and direction), full tile.
       Choice sc;
-      if (!h->force_generic &&
+      const bool chosen =
+          !h->force_generic &&
           choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, false, &sc, 0) ==
-              B200FFT_SUCCESS &&
-          sc.family == 0) {
+              B200FFT_SUCCESS;
+      // A pass with a compiled mixed-length kernel but no grouped form of it
+      // launches on its own.
+      const bool mixed = chosen && sc.mixed.one != nullptr;
+      if (mixed && sc.mixed.group == nullptr) {
+        const long long total = p.batch * op.slabs;
+        GroupStep s;
+        s.type = GroupStep::SINGLE;
+        s.f64 = f64s;
+        s.kind = p.kind;
+        s.col = sc.col;
+        s.fwd = fwds;
+        s.L = sc.L;
+        s.h = h;
+        s.plan = p;
+        s.plan.ch = sc;
+        s.dir = op.dir;
+        s.pa = pass_args(p, sc.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
+        s.sitems.push_back(s.pa);
+        s.bytes = pass_bytes(h, p, total);
+        g->steps.push_back(s);
+        continue;
+      }
+      if (mixed || (chosen && sc.family == 0)) {
+        const bool odd = mixed && sc.family == 1 && sc.gen.odd;
         const long long key = (1ll << 40) | (static_cast<long long>(sc.L) << 8) |
                               (f64s ? 1 : 0) | (p.kind << 1) | ((sc.col ? 1 : 0) << 3) |
-                              ((fwds ? 1 : 0) << 4);
+                              ((fwds ? 1 : 0) << 4) | ((odd ? 1 : 0) << 5);
         auto it = bucket.find(key);
         size_t si;
         if (it == bucket.end()) {
@@ -2006,6 +2060,8 @@ int group_build(G *g) {
           s.col = sc.col;
           s.fwd = fwds;
           s.L = sc.L;
+          if (mixed)
+            s.mixed = sc.mixed;
           s.tile_start.push_back(0);
           g->steps.push_back(s);
           si = g->steps.size() - 1;
@@ -2014,14 +2070,17 @@ int group_build(G *g) {
           si = it->second;
         }
         GroupStep &s = g->steps[si];
-        const PassArgs pa = pass_args(p, 0, op.in, op.out, op.tw, op.slabs, op.slab);
+        const PassArgs pa =
+            pass_args(p, sc.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
         if (s.sitems.empty()) {
           s.h = h;
           s.plan = p;
           s.dir = op.dir;
-          s.pa = pass_args(p, p.ch.family, op.in, op.out, op.tw, op.slabs, op.slab);
+          s.pa = pass_args(p, p.ch.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
         }
-        const int tb = static_tile_transforms(h->csize(), sc.L, sc.col);
+        const int csz = static_cast<int>(h->csize());
+        const int tb = mixed ? mixed_plan(sc.L, csz, sc.col).TB
+                             : static_tile_transforms(csz, sc.L, sc.col);
         s.sitems.push_back(pa);
         s.tile_start.push_back(s.tile_start.back() + (pa.total + tb - 1) / tb);
         s.bytes += pass_bytes(h, p, pa.total);
@@ -2030,7 +2089,7 @@ int group_build(G *g) {
       Choice gc;
       B2_TRY(choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, true, &gc));
       GenArgs ga = gc.gen;
-      ga.p = pass_args(p, 1, op.in, op.out, op.tw, op.slabs, op.slab);
+      ga.p = pass_args(p, false, op.in, op.out, op.tw, op.slabs, op.slab);
       const bool f64 = h->prec == B200FFT_F64;
       const bool fwd = op.dir == B200FFT_FORWARD;
       const int key = (f64 ? 1 : 0) | (p.kind << 1) | ((gc.col ? 1 : 0) << 3) | ((fwd ? 1 : 0) << 4);
@@ -2250,7 +2309,9 @@ int group_run(G *g) {
       } else if (s.type == GroupStep::STATIC) {
         what = "grouped specialised pass";
         const long long nt = s.tile_start.back();
-        if (s.kind == KIND_C2C)
+        if (s.mixed.group != nullptr)
+          e = s.mixed.group(s.d_sitems, s.d_tile_map, nt, s.fwd ? 0u : 0x80000000u, st);
+        else if (s.kind == KIND_C2C)
           e = s.f64 ? launch_static_group_c2c_f64(s.L, s.col, s.fwd, s.d_sitems, s.d_tile_map,
                                                   nt, st)
                     : launch_static_group_c2c_f32(s.L, s.col, s.fwd, s.d_sitems, s.d_tile_map,

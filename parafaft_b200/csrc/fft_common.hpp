@@ -384,13 +384,11 @@ constexpr int floor_pow2(int x) {
 
 constexpr CfgS cfg_static(int esize, int L, bool col, int variant = 0) {
   if (!is_pow2(L)) {
-    // Mixed-radix lengths (factors 8, 4, 2, 5, 3): power-of-two tiles and
-    // thread counts per transform; columns also take the half tile (variant
-    // 1: 10-15 points per thread, more CTAs per SM).
+    // Mixed-radix lengths (factors 8, 4, 2, 5, 3) in the group schedule kernel:
+    // power-of-two tiles and thread counts per transform.
     const int NT = 256;
-    const int base = esize == 8 ? 8192 : 4096;
+    const int tile = esize == 8 ? 8192 : 4096;
     if (col) {
-      const int tile = base >> (variant == 1 ? 1 : 0);
       const int TB = ce_min(NT, floor_pow2(ce_max(1, tile / L)));
       return CfgS{NT, TB, NT / TB, (TB * L + NT - 1) / NT};
     }
@@ -442,8 +440,9 @@ constexpr CfgS cfg_static(int esize, int L, bool col, int variant = 0) {
 }
 
 // Lengths with a specialised kernel (complex points of the stage loop):
-// powers of two up to 4096, and the mixed-radix lengths below (the sides of
-// common non-power-of-two grids and their R2C halves).
+// powers of two up to 4096, and the mixed-radix lengths below, which run the
+// compiled plans of mixed_plan.hpp (the group schedule kernel keeps tiles of
+// its own for them).
 constexpr int kStaticMaxL = 4096;
 constexpr bool static_pow2_ok(int L) { return L >= 2 && L <= kStaticMaxL && is_pow2(L); }
 constexpr bool static_mixed_ok(int L) {

@@ -71,6 +71,21 @@ bool colpair_length_ok(int L);
 bool colpair_vec_ok(const PassArgs &a);
 cudaError_t launch_colpair_c2c_f32(int L, bool fwd, const PassArgs &a, cudaStream_t st);
 
+// Family M: kernels compiled for lengths with odd prime factors (fft_mixed.cuh;
+// mixed_length_ok in mixed_plan.hpp). The launchers of one length, or nulls.
+// C2C kernels take flip = 0 (forward) or 0x80000000 (backward); R2C/C2R ones
+// ignore it. `a` is in complex units on both sides, except that the real side
+// of an odd length is in reals (rows contiguous in both).
+// group: the passes of many grids, items and tile map as for the grouped
+// Family S passes (tiles of mixed_plan(...).TB transforms); lengths up to
+// kMixedGroupMaxL have it.
+struct MixedKernel {
+  cudaError_t (*one)(const PassArgs &a, unsigned flip, cudaStream_t st) = nullptr;
+  cudaError_t (*group)(const PassArgs *items, const int2 *tile_map, long long ntiles,
+                       unsigned flip, cudaStream_t st) = nullptr;
+};
+MixedKernel mixed_kernel(bool f64, int kind, bool odd, bool col, int L);
+
 // Family G: runtime-generic kernels.
 cudaError_t launch_generic(bool f64, int kind, bool col, bool fwd,
                            const GenArgs &g, cudaStream_t st);
