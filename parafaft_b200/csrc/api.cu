@@ -256,7 +256,9 @@ int choose_kernel(int prec, int kind, int len, long long batch, long long stride
       !force_generic && static_length_ok(L) &&
       (kind == KIND_C2C || (!odd && stride == 1 && dist % 2 == 0 && L <= 2048));
   if (static_ok) {
-    int var = default_variant(csize, L, ch.col, stride);
+    const int tile = default_variant(csize, L, ch.col, stride);
+    const bool compiled_row = !ch.col && mixed_pow2_row(L, csize, kind != KIND_C2C);
+    int var = compiled_row ? kVariantCompiled : tile;
     if (const char *v = std::getenv("B200FFT_VARIANT")) {
       char *end = nullptr;
       const long ev = std::strtol(v, &end, 10);
@@ -274,7 +276,11 @@ int choose_kernel(int prec, int kind, int len, long long batch, long long stride
     }
     if (var == kVariantPair &&
         !(ch.col && kind == KIND_C2C && csize == 8 && colpair_length_ok(L)))
-      var = default_variant(csize, L, ch.col, stride); // the pair tile does not apply
+      var = tile; // the pair tile does not apply
+    if (var == kVariantCompiled && !compiled_row)
+      var = tile;
+    if (var == kVariantCompiled)
+      ch.mixed = mixed_kernel(prec == B200FFT_F64, kind, odd, false, L);
     const CfgS c = cfg_static(csize, L, ch.col, var);
     ch.variant = var;
     ch.family = 0;
@@ -1085,6 +1091,7 @@ int autotune(H *h, Plan &p) {
       const int nv = rigor >= B200FFT_PLAN_PATIENT ? 3 : 2;
       for (int v = 0; v < nv; ++v)
         cands.push_back({0, v});
+      cands.push_back({0, kVariantCompiled});
     }
   }
   if (rigor >= B200FFT_PLAN_PATIENT || p.ch.family == 1)
@@ -2021,7 +2028,7 @@ int group_build(G *g) {
       Choice sc;
       const bool chosen =
           !h->force_generic &&
-          choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, false, &sc, 0) ==
+          choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, false, &sc) ==
               B200FFT_SUCCESS;
       // A pass with a compiled mixed-length kernel but no grouped form of it
       // launches on its own.

@@ -366,9 +366,12 @@ struct CfgS {
 //  10 = pair-column tile (FP32, 256/512/1024 points): 512 (1024) threads, two
 //       neighbouring transforms per thread, 16-byte shared-memory exchanges
 //       and twiddles shared by the pair (fft_colpair.cuh).
-// Where a TMA or pair variant does not apply, the plan's default tile runs
-// instead.
-constexpr int kStaticVariants = 11;
+//  11 = compiled plan of a power-of-two row (mixed_pow2_row in mixed_plan.hpp):
+//       the kernels of the mixed lengths; the default where it exists.
+// Where a TMA, pair or compiled variant does not apply, the plan's default tile
+// runs instead.
+constexpr int kStaticVariants = 12;
+constexpr int kVariantCompiled = 11;
 constexpr int kVariantTma = 8;
 constexpr int kVariantPair = 10;
 constexpr int kVariantStaged = 4;

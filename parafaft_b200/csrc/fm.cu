@@ -10,14 +10,16 @@ namespace b200fft {
   MixedKernel fm_##p##_##f##_1(int L, int kind);                               \
   MixedKernel fm_##p##_##f##_2(int L, int kind);                               \
   MixedKernel fm_##p##_##f##_3(int L, int kind);                               \
+  MixedKernel fm_##p##_##f##_4(int L, int kind);                               \
   static MixedKernel find_##p##_##f(int L, int kind) {                         \
     return L < kMixedCut[0]   ? fm_##p##_##f##_0(L, kind)                      \
            : L < kMixedCut[1] ? fm_##p##_##f##_1(L, kind)                      \
            : L < kMixedCut[2] ? fm_##p##_##f##_2(L, kind)                      \
-                              : fm_##p##_##f##_3(L, kind);                     \
+           : L < kMixedCut[3] ? fm_##p##_##f##_3(L, kind)                      \
+                              : fm_##p##_##f##_4(L, kind);                     \
   }
 // ranges of lengths of the compilation units (FM_LO / FM_HI in build.py)
-static constexpr int kMixedCut[3] = {136, 351, 801};
+static constexpr int kMixedCut[4] = {136, 351, 801, 2049};
 FM_DECLARE(32, 0)
 FM_DECLARE(32, 1)
 FM_DECLARE(32, 2)
@@ -27,7 +29,10 @@ FM_DECLARE(64, 2)
 
 // L: complex points of the stage loop (n/2 for an even real length n, else n).
 MixedKernel mixed_kernel(bool f64, int kind, bool odd, bool col, int L) {
-  if (!mixed_length_ok(L, col) || (kind != KIND_C2C && col))
+  if (kind != KIND_C2C && col)
+    return MixedKernel{};
+  if (!mixed_length_ok(L, col) &&
+      (col || !mixed_pow2_row(L, f64 ? 16 : 8, kind != KIND_C2C)))
     return MixedKernel{};
   if (kind == KIND_C2C)
     return f64 ? (col ? find_64_0(L, kind) : find_64_1(L, kind))

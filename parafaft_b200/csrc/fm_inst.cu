@@ -80,11 +80,11 @@ template <int L> constexpr MixedKernel entry(int kind) {
   if constexpr (mixed_length_ok(L, true))
     return kernel<L, KIND_C2C, false, true>();
 #elif FM_FORM == 1
-  if constexpr (mixed_length_ok(L, false))
+  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), false))
     return kernel<L, KIND_C2C, false, false>();
 #else
   // kind: KIND_R2C or KIND_C2R of real length 2L, or of odd length L (| 4)
-  if constexpr (mixed_length_ok(L, false)) {
+  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), true)) {
     if (kind == KIND_R2C)
       return kernel<L, KIND_R2C, false, false>();
     if (kind == KIND_C2R)

@@ -199,3 +199,33 @@ def test_measured_plans_keep_the_compiled_kernel():
         h.plan_c2c(0, 100, 64, 64, 1)
         assert h.plan_describe(nv.KIND_C2C, 0).count("compiled=") == 1
     nv.forget_wisdom()
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("length", [8, 16, 32, 64, 128, 256, 512, 2048, 4096])
+def test_compiled_power_of_two_rows(prec, length):
+    """Rows of powers of two on compiled plans: batches around the tile, both
+    directions, and R2C/C2R of twice the length."""
+    d = nv.describe(prec, nv.KIND_C2C, length)
+    tb = re.search(r"on \d+x(\d+) threads", d)
+    tb = int(tb.group(1)) if tb else 4
+    for batch in {1, max(1, tb - 1), tb, tb + 1, 3 * tb + 1}:
+        for direction in (nv.FORWARD, nv.BACKWARD):
+            y, ref, _ = _c2c(prec, length, batch, 1, length, direction)
+            assert O.rel_l2(y, ref) < tol(prec), (length, batch, d)
+        if length > 2048:
+            continue
+        n, nc = 2 * length, length + 1
+        x = O.normal_real((batch, n), batch).astype(rdtype(prec))
+        h = nv.Handle(prec, 0)
+        h.plan_r2c(n, batch, 1, 2 * nc)
+        h.plan_c2r(n, batch, 1, 2 * nc)
+        buf = to_dev(O.pad_real(x, rdtype(prec)))
+        h.exec_r2c(buf)
+        h.sync()
+        X = to_host(buf).view(cdtype(prec)).reshape(batch, nc)
+        assert O.rel_l2(X, np.stack([O.r2c_nd(r) for r in x.astype(np.float64)])) < tol(prec)
+        h.exec_c2r(buf)
+        h.sync()
+        back = to_host(buf).reshape(batch, 2 * nc)[:, :n]
+        assert O.rel_l2(back / n, x) < tol(prec), (n, batch)
