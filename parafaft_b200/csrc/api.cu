@@ -855,21 +855,37 @@ int device_sms(int dev) {
 // SM two full tiles (e.g. a 64^3 grid) takes the half or quarter tile, so more
 // CTAs share its latency. Only the Estimate default is adjusted; measured
 // plans keep their choice.
-int column_tile_for(const H *h, const Plan &p, long long total) {
-  int var = p.ch.variant;
-  if (h->plan_flag != B200FFT_PLAN_ESTIMATE || !p.ch.col || !is_pow2(p.ch.L) ||
-      (var != 0 && var != 5))
+int column_tile(int csz, int L, int var, long long total, int sms) {
+  if (var != 0 && var != 5)
     return var;
-  const long long want = 2ll * device_sms(h->device);
-  const int csz = h->csize();
-  if ((total + cfg_static(csz, p.ch.L, true, var).TB - 1) / cfg_static(csz, p.ch.L, true, var).TB >=
-      want)
+  const long long want = 2ll * sms;
+  const auto tiles = [&](int v) {
+    const int tb = cfg_static(csz, L, true, v).TB;
+    return (total + tb - 1) / tb;
+  };
+  if (tiles(var) >= want)
     return var;
   for (int v = 1; v <= 2; ++v)
-    if ((total + cfg_static(csz, p.ch.L, true, v).TB - 1) / cfg_static(csz, p.ch.L, true, v).TB >=
-        want)
+    if (tiles(v) >= want)
       return v;
   return 2;
+}
+
+int column_tile_for(const H *h, const Plan &p, long long total) {
+  if (h->plan_flag != B200FFT_PLAN_ESTIMATE || !p.ch.col || !is_pow2(p.ch.L))
+    return p.ch.variant;
+  return column_tile(static_cast<int>(h->csize()), p.ch.L, p.ch.variant, total,
+                     device_sms(h->device));
+}
+
+// FP32 512-point columns whose neighbouring transforms sit side by side on
+// 16-byte aligned rows (the first axis of a grid) take the pair tile by default:
+// 16-byte loads, stores and exchanges (512^3 first-axis pass 0.212 -> 0.195
+// ms); odd point strides keep the one-transform tile (the pair tile's 8-byte
+// form was slower there, 0.237 vs 0.225 ms, and so was the TMA double-row
+// kernel, 0.235 ms).
+bool pair_by_default(bool f64, int L, int var, const PassArgs &a) {
+  return var == 5 && !f64 && L == 512 && colpair_vec_ok(a);
 }
 
 cudaError_t launch_kernel(H *h, const Plan &p, int dir, const PassArgs &a) {
@@ -881,14 +897,8 @@ cudaError_t launch_kernel(H *h, const Plan &p, int dir, const PassArgs &a) {
   } else if (p.ch.family == 0) {
     if (p.kind == KIND_C2C) {
       int var = column_tile_for(h, p, a.total);
-      // FP32 512-point columns whose neighbouring transforms sit side by side
-      // on 16-byte aligned rows (the first axis of a grid) take the pair tile
-      // by default: 16-byte loads, stores and exchanges (512^3 first-axis
-      // pass 0.212 -> 0.195 ms); odd point strides keep the one-transform
-      // tile (the pair tile's 8-byte form was slower there, 0.237 vs 0.225 ms,
-      // and so was the TMA double-row kernel, 0.235 ms)
-      if (var == 5 && h->plan_flag == B200FFT_PLAN_ESTIMATE && !f64 && p.ch.col &&
-          p.ch.L == 512 && colpair_vec_ok(a))
+      if (h->plan_flag == B200FFT_PLAN_ESTIMATE && p.ch.col &&
+          pair_by_default(f64, p.ch.L, var, a))
         var = kVariantPair;
       if (var == kVariantPair && !f64 && p.ch.col && colpair_length_ok(p.ch.L))
         return launch_colpair_c2c_f32(p.ch.L, fwd, a, h->stream);
@@ -931,6 +941,29 @@ cudaError_t launch_kernel(H *h, const Plan &p, int dir, const PassArgs &a) {
   }
   return e;
 }
+
+} // namespace
+
+namespace b200fft {
+cudaError_t launch_default_c2c(bool f64, int L, bool col, bool fwd, const PassArgs &a,
+                               cudaStream_t st) {
+  const int csz = f64 ? 16 : 8;
+  if (!col && mixed_pow2_row(L, csz, false))
+    return mixed_kernel(f64, KIND_C2C, false, false, L).one(a, fwd ? 0u : 0x80000000u, st);
+  int var = default_variant(csz, L, col, a.istride);
+  if (col) {
+    int dev = -1;
+    cudaGetDevice(&dev);
+    var = column_tile(csz, L, var, a.total, device_sms(dev));
+    if (pair_by_default(f64, L, var, a))
+      return launch_colpair_c2c_f32(L, fwd, a, st);
+  }
+  return f64 ? launch_static_c2c_f64(L, col, fwd, var, a, st)
+             : launch_static_c2c_f32(L, col, fwd, var, a, st);
+}
+} // namespace b200fft
+
+namespace {
 
 int flush_run(H *h) {
   if (!h->run.active)

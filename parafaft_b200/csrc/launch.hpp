@@ -86,6 +86,10 @@ struct MixedKernel {
 };
 MixedKernel mixed_kernel(bool f64, int kind, bool odd, bool col, int L);
 
+// The kernel of an Estimate plan of a power-of-two C2C pass (api.cu).
+cudaError_t launch_default_c2c(bool f64, int L, bool col, bool fwd, const PassArgs &a,
+                               cudaStream_t st);
+
 // Family G: runtime-generic kernels.
 cudaError_t launch_generic(bool f64, int kind, bool col, bool fwd,
                            const GenArgs &g, cudaStream_t st);

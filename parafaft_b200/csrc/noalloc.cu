@@ -9,27 +9,28 @@
 // use this entry point instead.
 //
 // How: the one piece of memory the transform needs besides its input and
-// output, the twiddle table, lives in a fixed array in the library's own
-// device image (8192 complex doubles, 128 KiB, held on every device that loads
-// the library until the process exits). Each call rewrites the table for its
-// length in that array and then runs the specialised C2C kernel on the
-// caller's stream; nothing in the array has to start at zero.
+// output, the twiddle table, lives in fixed arrays in the library's own device
+// image (8191 entries per precision, 192 KiB, held on every device that loads
+// the library until the process exits). They hold the table pyramid of 4096
+// points, whose levels are the tables of every shorter power of two: one fill
+// per device and precision serves all lengths, and a call is one kernel. (A
+// fill before every transform made each call two dependent kernels: forward and
+// backward of 512 columns of 128 FP32 points 20.5 us; 13.5 us without it.)
 //
 // Limits and rules for callers:
-//  * lengths are powers of two from 2 to 4096 (the array's capacity); other
+//  * lengths are powers of two from 2 to 4096 (the arrays' capacity); other
 //    lengths are rejected with B200FFT_ERR_UNSUPPORTED before any GPU work;
-//  * the first call on a device looks up the array's device address with
-//    cudaGetSymbolAddress (once per device, with that device current); make
-//    that first call before any stream capture begins;
-//  * the address is kept for the life of the process: calls after
+//  * the first call on a device looks up the arrays' device addresses with
+//    cudaGetSymbolAddress (once per device, with that device current), and the
+//    first call of a precision fills its table on the caller's stream; make
+//    these before any stream capture begins (a capture that comes first fills
+//    the table inside the captured work, at every replay);
+//  * the addresses are kept for the life of the process: calls after
 //    cudaDeviceReset on that device are not supported (the module, and with
-//    it the array, may move);
-//  * the transform runs the specialised kernel's default tile (variant 0)
-//    whatever the stride; a handle's plan may pick a wider column tile;
-//  * every call on a device shares the one array and leaves its table there:
-//    two calls that can run at the same time on the GPU (different streams
-//    without ordering between them) race on it. Order them on one stream or
-//    with events.
+//    it the arrays, may move);
+//  * the transform runs the kernel an Estimate plan of the same shape takes;
+//  * calls on different streams need no ordering among themselves: until the
+//    fill has finished, calls on other streams wait for it (on the device).
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -45,29 +46,35 @@ void set_error_text(const std::string &msg); // api.cu: text of b200fft_last_err
 
 #define NOALLOC_MAX_LENGTH 4096
 
-// The twiddle table of b200fft_c2c_noalloc: 2 * NOALLOC_MAX_LENGTH complex
-// doubles (128 KiB), room for the table pyramid of the longest length. Host
-// code must not pass this name to a kernel: on the host it only stands for the
-// symbol. The device address comes from cudaGetSymbolAddress (device_table
+// The table pyramids of NOALLOC_MAX_LENGTH points, FP64 and FP32. Host code
+// must not pass these names to a kernel: on the host they only stand for the
+// symbols. The device addresses come from cudaGetSymbolAddress (device_table
 // below).
-static __device__ __align__(256) unsigned char g_noalloc_table[2 * NOALLOC_MAX_LENGTH * 16];
+static __device__ __align__(256) unsigned char g_noalloc_table64[2 * NOALLOC_MAX_LENGTH * 16];
+static __device__ __align__(256) unsigned char g_noalloc_table32[2 * NOALLOC_MAX_LENGTH * 8];
 
 namespace {
 
 constexpr int kNoAllocMaxLength = NOALLOC_MAX_LENGTH;
 constexpr int kMaxDevices = 64;
 
+// One precision's table on one device.
+struct Table {
+  void *addr = nullptr;
+  bool filled = false;         // the fill has finished on the device
+  cudaEvent_t fill = nullptr;  // recorded after the fill until then
+};
 std::mutex g_mu;
-void *g_table_addr[kMaxDevices] = {nullptr};
+Table g_tables[kMaxDevices][2];
 
 int fail(int code, const std::string &msg) {
   b200fft::set_error_text(msg);
   return code;
 }
 
-// Device address of g_noalloc_table on the current device, resolved once per
-// device with that device current.
-int device_table(void **out) {
+// The current device's table of one precision, ready for work that `st` runs
+// from now on.
+int device_table(bool f64, cudaStream_t st, void **out) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -75,16 +82,50 @@ int device_table(void **out) {
                 std::string("b200fft_c2c_noalloc: no usable current device: ") +
                     cudaGetErrorString(e));
   std::lock_guard<std::mutex> lk(g_mu);
-  if (g_table_addr[dev] == nullptr) {
+  Table &t = g_tables[dev][f64 ? 1 : 0];
+  if (t.addr == nullptr) {
     void *p = nullptr;
-    e = cudaGetSymbolAddress(&p, g_noalloc_table);
+    e = f64 ? cudaGetSymbolAddress(&p, g_noalloc_table64)
+            : cudaGetSymbolAddress(&p, g_noalloc_table32);
     if (e != cudaSuccess || p == nullptr)
       return fail(B200FFT_ERR_CUDA,
                   std::string("b200fft_c2c_noalloc: cudaGetSymbolAddress failed: ") +
                       cudaGetErrorString(e));
-    g_table_addr[dev] = p;
+    t.addr = p;
   }
-  *out = g_table_addr[dev];
+  *out = t.addr;
+  if (t.filled)
+    return B200FFT_SUCCESS;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  e = cudaStreamIsCapturing(st, &cap);
+  if (e != cudaSuccess) { // the legacy stream while another stream captures
+    cudaGetLastError();
+    cap = cudaStreamCaptureStatusActive;
+  }
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
+  if (!capturing && t.fill != nullptr) {
+    if (cudaEventQuery(t.fill) == cudaSuccess) {
+      t.filled = true;
+      cudaEventDestroy(t.fill);
+      t.fill = nullptr;
+      return B200FFT_SUCCESS;
+    }
+    cudaGetLastError(); // not ready yet
+    e = cudaStreamWaitEvent(st, t.fill, 0);
+  } else {
+    e = f64 ? b200fft::launch_twiddle_table(static_cast<double2 *>(t.addr), nullptr,
+                                            kNoAllocMaxLength, st)
+            : b200fft::launch_twiddle_table(nullptr, static_cast<float2 *>(t.addr),
+                                            kNoAllocMaxLength, st);
+    if (e == cudaSuccess && !capturing) {
+      e = cudaEventCreateWithFlags(&t.fill, cudaEventDisableTiming);
+      if (e == cudaSuccess)
+        e = cudaEventRecord(t.fill, st);
+    }
+  }
+  if (e != cudaSuccess)
+    return fail(B200FFT_ERR_CUDA,
+                std::string("b200fft_c2c_noalloc: twiddle table: ") + cudaGetErrorString(e));
   return B200FFT_SUCCESS;
 }
 
@@ -111,32 +152,25 @@ extern "C" int b200fft_c2c_noalloc(int precision, int direction, int length, siz
   if (batch > (1ull << 40) || stride > (1ll << 44) || dist > (1ll << 44))
     return fail(B200FFT_ERR_RANGE,
                 "b200fft_c2c_noalloc: batch/stride/dist exceed the supported range");
-  void *table = nullptr;
-  int rc = device_table(&table);
-  if (rc != B200FFT_SUCCESS)
-    return rc;
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const bool f64 = precision == B200FFT_F64;
-  // The whole table for this length is rewritten, so nothing left by an
-  // earlier call is read.
-  cudaError_t e = f64 ? launch_twiddle_table(static_cast<double2 *>(table), nullptr, length, st)
-                      : launch_twiddle_table(nullptr, static_cast<float2 *>(table), length, st);
-  if (e != cudaSuccess)
-    return fail(B200FFT_ERR_CUDA,
-                std::string("b200fft_c2c_noalloc: twiddle kernel: ") + cudaGetErrorString(e));
+  void *table = nullptr;
+  const int rc = device_table(f64, st, &table);
+  if (rc != B200FFT_SUCCESS)
+    return rc;
+  // level `length` of the pyramid: its table and those of the shorter lengths
+  const size_t level = static_cast<size_t>(2 * kNoAllocMaxLength - 2 * length);
   PassArgs a{};
   a.in = in;
   a.out = out;
-  a.tw = table;
+  a.tw = static_cast<const char *>(table) + level * (f64 ? sizeof(double2) : sizeof(float2));
   a.total = static_cast<long long>(batch);
   a.batch = static_cast<long long>(batch);
   a.idist = a.odist = dist;
   a.istride = a.ostride = stride;
   a.islab = a.oslab = 0;
-  const bool col = dist < stride;
-  const bool fwd = direction == B200FFT_FORWARD;
-  e = f64 ? launch_static_c2c_f64(length, col, fwd, 0, a, st)
-          : launch_static_c2c_f32(length, col, fwd, 0, a, st);
+  const cudaError_t e = launch_default_c2c(f64, length, dist < stride,
+                                           direction == B200FFT_FORWARD, a, st);
   if (e != cudaSuccess)
     return fail(B200FFT_ERR_CUDA,
                 std::string("b200fft_c2c_noalloc: transform kernel: ") + cudaGetErrorString(e));
