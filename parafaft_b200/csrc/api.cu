@@ -2072,14 +2072,13 @@ int group_build(G *g) {
         s.type = GroupStep::SINGLE;
         s.f64 = f64s;
         s.kind = p.kind;
-        s.col = sc.col;
+        s.col = p.ch.col;
         s.fwd = fwds;
-        s.L = sc.L;
+        s.L = p.ch.L;
         s.h = h;
-        s.plan = p;
-        s.plan.ch = sc;
+        s.plan = p; // its own choice: split-precision and tuned plans keep theirs
         s.dir = op.dir;
-        s.pa = pass_args(p, sc.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
+        s.pa = pass_args(p, p.ch.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
         s.sitems.push_back(s.pa);
         s.bytes = pass_bytes(h, p, total);
         g->steps.push_back(s);

@@ -229,3 +229,27 @@ def test_compiled_power_of_two_rows(prec, length):
         h.sync()
         back = to_host(buf).reshape(batch, 2 * nc)[:, :n]
         assert O.rel_l2(back / n, x) < tol(prec), (n, batch)
+
+
+def test_grouped_split_precision_rows_keep_their_kernel():
+    """A group's pass that launches alone runs its plan's own kernel: 512-point
+    split-precision rows give the bits they give outside a group."""
+    n, b = 512, 33
+    x = O.normal_complex(n * b, 7).astype(np.complex64)
+    outs = []
+    for grouped in (False, True):
+        h = nv.Handle(nv.F32, 1, flags=nv.FLAG_SPLIT_TC)
+        h.plan_c2c(0, n, b, 1, n)
+        assert h.plan_describe(nv.KIND_C2C, 0).startswith("split-tc")
+        d = to_dev(x)
+        if grouped:
+            g = nv.Group([h])
+            g.begin()
+            h.exec_c2c(0, nv.FORWARD, d)
+            g.end()
+            g.sync()
+        else:
+            h.exec_c2c(0, nv.FORWARD, d)
+            h.sync()
+        outs.append(to_host(d))
+    assert np.array_equal(outs[0], outs[1])
