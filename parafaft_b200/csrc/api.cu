@@ -783,6 +783,18 @@ long long pass_bytes(const H *h, const Plan &p, long long total) {
   return total * (p.len * static_cast<long long>(h->rsize) + (p.len / 2 + 1) * cs);
 }
 
+// Whether a caller captures stream `st` into a graph: its passes then launch
+// without programmatic dependencies (the caller's fork and join events decide
+// the graph's edges).
+bool stream_captures(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError(); // the legacy stream while another stream captures
+    return true;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // in_dist >= 0 replaces the input row distance (in the kernel's input units):
 // the R2C pass of a fused pad reads the unpadded source rows.
 int launch_pass(H *h, const Plan &p, int dir, const void *in, void *out,
@@ -825,6 +837,7 @@ int launch_pass(H *h, const Plan &p, int dir, const void *in, void *out,
   }
   ProfileScope ps(h);
   h->last_tma = false;
+  a.chained = bytes <= kChainedBytes && !stream_captures(h->stream);
   const cudaError_t e = launch_kernel(h, p, dir, a);
   if (h->last_tma)
     r.family = 4;
@@ -2118,8 +2131,7 @@ int group_build(G *g) {
           s.pa = pass_args(p, p.ch.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
         }
         const int csz = static_cast<int>(h->csize());
-        const int tb = mixed ? mixed_plan(sc.L, csz, sc.col).TB
-                             : static_tile_transforms(csz, sc.L, sc.col);
+        const int tb = mixed ? sc.mixed.tb : static_tile_transforms(csz, sc.L, sc.col);
         s.sitems.push_back(pa);
         s.tile_start.push_back(s.tile_start.back() + (pa.total + tb - 1) / tb);
         s.bytes += pass_bytes(h, p, pa.total);
@@ -2313,6 +2325,7 @@ int group_run(G *g) {
     if (e != cudaSuccess)
       return cuda_fail(e, "group chain fork");
   }
+  size_t prev_width = 0; // steps of the level before (0: none yet)
   for (size_t lv = 0; lv < g->steps.size();) {
     size_t lv_end = lv;
     while (lv_end < g->steps.size() && g->steps[lv_end].level == g->steps[lv].level &&
@@ -2364,6 +2377,10 @@ int group_run(G *g) {
         what = "single pass";
         cudaStream_t keep = s.h->stream;
         s.h->stream = st; // the plan's launch goes to this step's stream
+        // a level of one pass after a level of one step, on one chain: the pass
+        // before is the kernel in front of it on the stream
+        s.pa.chained = g->chains == 1 && width == 1 && prev_width == 1 &&
+                       s.bytes <= kChainedBytes;
         e = launch_kernel(s.h, s.plan, s.dir, s.pa);
         s.h->stream = keep;
       } else if (s.type == GroupStep::COPY) {
@@ -2391,6 +2408,7 @@ int group_run(G *g) {
       if (e != cudaSuccess)
         return cuda_fail(e, "group level join");
     }
+    prev_width = width;
     lv = lv_end;
   }
   if (g->chains > 1) { // join: the group's stream waits for every chain

@@ -197,6 +197,7 @@ template <int L, int NT, int TB, bool FWD, bool VEC> struct KP {
     c.in1 = in + i1;
     c.out0 = out + o0;
     c.out1 = out + o1;
+    pass_begin(a);
     c.tw = reinterpret_cast<const V *>(a.tw);
     c.ist = a.istride;
     c.ost = a.ostride;

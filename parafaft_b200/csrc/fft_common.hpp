@@ -31,6 +31,9 @@ struct PassArgs {
   long long batch;    // transforms per slab
   long long idist, istride, islab;
   long long odist, ostride, oslab;
+  // The launch may overlap the drain of the kernel before it on its stream
+  // (launch_chained in launch.hpp, pass_begin in fft_device.cuh).
+  long long chained;
 };
 
 // Division by a runtime constant d < 2^31 for dividends n < 2^31:

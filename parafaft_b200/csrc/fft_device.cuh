@@ -45,6 +45,18 @@ template <bool FWD, typename V> BF_D V rot(V a) {
   return FWD ? cmake(a.y, -a.x) : cmake(-a.y, a.x);
 }
 
+// Start of a pass kernel that may be a programmatic dependent launch: let the
+// next kernel of the stream become resident as soon as every CTA of this one has
+// started, and touch no memory before the kernels in front have finished. The
+// launch and the CTAs' start-up then overlap the drain of the pass before: see
+// launch_chained for what that measured. Plain launches skip both.
+BF_D void pass_begin(const PassArgs &a) {
+  if (a.chained != 0) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+}
+
 BF_D uint32_t fdiv(uint32_t n, const FastDiv &f) {
   return f.m == 0 ? n : (__umulhi(n, f.m) >> f.s);
 }
@@ -393,6 +405,10 @@ struct KS {
   static constexpr int P = NT / TB; // threads per transform
   static constexpr int TSCALE = (KIND == KIND_C2C) ? 1 : 2;
   static constexpr bool WARP_SYNC = !COL && (P <= 32) && (32 % P == 0);
+  // FP32 passes may be programmatic dependent launches. FP64 ones are not: their
+  // columns run at the HBM peak, where even the untaken branch shows
+  // (64-point columns of a 128x128x64x64 grid 350 -> 360 us).
+  static constexpr bool CHAINS = sizeof(V) == 8;
   static_assert(NT % TB == 0, "TB must divide NT");
   static_assert(S.rest == 1, "length not factorable");
 
@@ -638,6 +654,8 @@ struct KS {
     c.ist = KIND == KIND_C2C ? a.istride : 1;
     c.ost = KIND == KIND_C2C ? a.ostride : 1;
     c.sm = sm;
+    if constexpr (CHAINS)
+      pass_begin(a);
 
     V v[EMAX];
     constexpr int R = S.rad[0];

@@ -496,6 +496,7 @@ struct KM {
     c.ost = a.ostride;
     c.flip = flip;
     c.sm = sm + (COL ? c.tb : c.tb * LP);
+    pass_begin(a);
     V v[EMAX];
     if constexpr (KIND == KIND_C2R && !ODD) {
       c2r_in(c);

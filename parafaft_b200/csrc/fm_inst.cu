@@ -47,8 +47,8 @@ cudaError_t launch_one(const PassArgs &a, unsigned flip, cudaStream_t st) {
     return cudaSuccess;
   if (grid > INT_MAX)
     return cudaErrorInvalidConfiguration;
-  fft_mixed_kernel<K><<<static_cast<unsigned>(grid), K::NT, K::smem_bytes(), st>>>(a, flip);
-  return cudaGetLastError();
+  return launch_chained(a.chained != 0, fft_mixed_kernel<K>, static_cast<unsigned>(grid), K::NT,
+                        K::smem_bytes(), st, a, flip);
 }
 
 template <int L, int KIND, bool ODD, bool COL>
@@ -69,7 +69,7 @@ cudaError_t launch_group(const PassArgs *items, const int2 *map, long long ntile
 }
 
 template <int L, int KIND, bool ODD, bool COL> constexpr MixedKernel kernel() {
-  MixedKernel k{&launch_one<L, KIND, ODD, COL>, nullptr};
+  MixedKernel k{&launch_one<L, KIND, ODD, COL>, nullptr, KM<Real, L, KIND, ODD, COL>::TB};
   if constexpr (L <= kMixedGroupMaxL)
     k.group = &launch_group<L, KIND, ODD, COL>;
   return k;

@@ -30,8 +30,7 @@ cudaError_t launch_colpair_one(const PassArgs &a, cudaStream_t st) {
     return cudaSuccess;
   if (grid > INT_MAX)
     return cudaErrorInvalidConfiguration;
-  kern<<<static_cast<unsigned>(grid), NT, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_chained(a.chained != 0, kern, static_cast<unsigned>(grid), NT, smem, st, a);
 }
 
 template <int L, int NT, int TB>

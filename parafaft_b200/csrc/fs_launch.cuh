@@ -35,8 +35,8 @@ cudaError_t launch_static_one(const PassArgs &a, cudaStream_t st) {
     return cudaSuccess;
   if (grid > INT_MAX)
     return cudaErrorInvalidConfiguration;
-  kern<<<static_cast<unsigned>(grid), cf.NT, smem, st>>>(a);
-  return cudaGetLastError();
+  return launch_chained(K::CHAINS && a.chained != 0, kern, static_cast<unsigned>(grid), cf.NT,
+                        smem, st, a);
 }
 
 inline int sm_count() {

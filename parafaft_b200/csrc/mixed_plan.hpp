@@ -47,7 +47,8 @@ constexpr bool mixed_length_ok(int L, bool col) {
 //     128 5.9 -> 6.3, 256 5.8 -> 6.4, 512 5.7 -> 6.0, 2048 4.3 -> 4.8,
 //     4096 4.2 -> 4.6 (1024 points 5.4 -> 5.3 stay);
 //   C2C FP64: 8 3.5 -> 5.6, 16 5.5 -> 6.5, 128 5.7 -> 6.2, 256 6.3 -> 6.4,
-//     2048 5.0 -> 5.2 (512, 1024 and 4096 stay: 6.2 -> 5.7, 5.1, 5.5 -> 4.8);
+//     2048 5.0 -> 5.2 (32, 64, 512, 1024 and 4096 stay: 6.5, 6.4, 6.2 -> 5.7, 5.1,
+//     5.5 -> 4.8);
 //   C2R FP32 of 2 x 16 3.5 -> 4.4, 2 x 128 5.4 -> 5.6, 2 x 1024 4.3 -> 5.1,
 //     2 x 2048 2.0 -> 3.8 (2 x 256 5.8 -> 5.6 stays);
 //   C2R FP64 of 2 x 16 4.5 -> 5.7, 2 x 64 5.7 -> 5.9, 2 x 1024 2.8 -> 4.0,
@@ -57,7 +58,8 @@ constexpr bool mixed_pow2_row(int L, int es, bool real) {
     return false;
   if (real)
     return L <= 2048 && !(es == 8 && L == 256) && !(es == 16 && L == 512);
-  return es == 8 ? L <= 4096 && L != 1024 : L <= 2048 && L != 512 && L != 1024;
+  return es == 8 ? L <= 4096 && L != 1024
+                 : L <= 2048 && L != 32 && L != 64 && L != 512 && L != 1024;
 }
 
 constexpr int ce_div_up(int a, int b) { return (a + b - 1) / b; }

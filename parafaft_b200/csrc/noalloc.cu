@@ -169,6 +169,13 @@ extern "C" int b200fft_c2c_noalloc(int precision, int direction, int length, siz
   a.idist = a.odist = dist;
   a.istride = a.ostride = stride;
   a.islab = a.oslab = 0;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError(); // the legacy stream while another stream captures
+    cap = cudaStreamCaptureStatusActive;
+  }
+  a.chained = cap == cudaStreamCaptureStatusNone && // as a handle's passes
+              2 * a.total * length * (f64 ? 16 : 8) <= kChainedBytes;
   const cudaError_t e = launch_default_c2c(f64, length, dist < stride,
                                            direction == B200FFT_FORWARD, a, st);
   if (e != cudaSuccess)
