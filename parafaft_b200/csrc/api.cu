@@ -187,9 +187,10 @@ int default_variant(int csize, int L, bool col, long long stride) {
     // (FP32: 32 points per thread, two 32-point stages)
     if (L == 1024)
       return stride * csize >= (4ll << 20) ? 3 : 0;
-    // FP32 columns of 128-512 points: 512-thread full tiles, two CTAs per SM
-    // (at 4 MiB strides 128/256 points 6.1 TB/s vs 4.5-5.0 for the other tiles)
-    if (csize == 8 && L >= 128)
+    // FP32 columns of 64-512 points: 512-thread full tiles, two CTAs per SM (at 4
+    // MiB strides 128/256 points 6.1 TB/s vs 4.5-5.0 for the other tiles; 400 MB
+    // of 64 points 5.9 against 5.3 for the 256-thread full tile)
+    if (csize == 8 && L >= kWideThreadsMinL)
       return 5;
     // FP64 columns of 512 points or fewer: the full tile at any stride
     // (256 points at a 4 MiB stride 6.4 vs 4.7 TB/s for the wide tile)

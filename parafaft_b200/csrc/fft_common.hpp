@@ -375,6 +375,8 @@ struct CfgS {
 // runs instead.
 constexpr int kStaticVariants = 12;
 constexpr int kVariantCompiled = 11;
+// FP32 columns from this length on run full tiles on 512 threads (variant 5).
+constexpr int kWideThreadsMinL = 64;
 constexpr int kVariantTma = 8;
 constexpr int kVariantPair = 10;
 constexpr int kVariantStaged = 4;

@@ -136,11 +136,16 @@ cudaError_t launch_static_var(int var, const PassArgs &a, cudaStream_t st) {
   }
 }
 
-// Grouped specialised pass (full tile): one CTA per tile of every item.
+// Grouped specialised pass (full tile): one CTA per tile of every item. FP32
+// columns of 64-512 points take its 512-thread form, as single passes do (the
+// same transforms per tile).
 template <typename T, int L, bool COL, bool FWD, int KIND>
 cudaError_t launch_static_group_one(const PassArgs *items, const int2 *tile_map, long long ntiles,
                                     cudaStream_t st) {
-  constexpr CfgS cf = cfg_static(static_cast<int>(sizeof(cvec<T>)), L, COL, 0);
+  constexpr int ES = static_cast<int>(sizeof(cvec<T>));
+  constexpr int VAR = COL && ES == 8 && L >= kWideThreadsMinL && L <= 512 ? 5 : 0;
+  constexpr CfgS cf = cfg_static(ES, L, COL, VAR);
+  static_assert(cf.TB == cfg_static(ES, L, COL, 0).TB, "static_tile_transforms");
   using K = KS<T, L, cf.NT, cf.TB, COL, FWD, KIND>;
   auto kern = fft_static_group_kernel<T, L, cf.NT, cf.TB, COL, FWD, KIND>;
   constexpr size_t smem = K::smem_bytes();
