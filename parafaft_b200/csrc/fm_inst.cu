@@ -75,7 +75,8 @@ template <int L, int KIND, bool ODD, bool COL> constexpr MixedKernel kernel() {
   return k;
 }
 
-template <int L> constexpr MixedKernel entry(int kind) {
+// KINDX: KIND_C2C; KIND_R2C or KIND_C2R of real length 2L, or of odd length L (| 4).
+template <int L, int KINDX> constexpr MixedKernel entry() {
 #if FM_FORM == 0
   if constexpr (mixed_length_ok(L, true))
     return kernel<L, KIND_C2C, false, true>();
@@ -83,31 +84,42 @@ template <int L> constexpr MixedKernel entry(int kind) {
   if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), false))
     return kernel<L, KIND_C2C, false, false>();
 #else
-  // kind: KIND_R2C or KIND_C2R of real length 2L, or of odd length L (| 4)
   if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), true)) {
-    if (kind == KIND_R2C)
-      return kernel<L, KIND_R2C, false, false>();
-    if (kind == KIND_C2R)
-      return kernel<L, KIND_C2R, false, false>();
-    if constexpr (L % 2 == 1)
-      return kind == (KIND_R2C | 4) ? kernel<L, KIND_R2C, true, false>()
-                                    : kernel<L, KIND_C2R, true, false>();
+    if constexpr ((KINDX & 4) == 0)
+      return kernel<L, KINDX, false, false>();
+    else if constexpr (L % 2 == 1)
+      return kernel<L, KINDX & 3, true, false>();
   }
 #endif
   return MixedKernel{};
 }
 
-template <int... I>
-MixedKernel find(int L, int kind, std::integer_sequence<int, I...>) {
-  MixedKernel f{};
-  ((L == FM_LO + I ? (f = entry<FM_LO + I>(kind), true) : false) || ...);
-  return f;
+template <int KINDX, int... I>
+const MixedKernel *table(std::integer_sequence<int, I...>) {
+  static const MixedKernel t[] = {entry<FM_LO + I, KINDX>()...};
+  return t;
+}
+template <int KINDX> MixedKernel find(int L) {
+  return table<KINDX>(std::make_integer_sequence<int, FM_HI - FM_LO>{})[L - FM_LO];
 }
 
 } // namespace
 
 MixedKernel FM_NAME(int L, int kind) {
-  return find(L, kind, std::make_integer_sequence<int, FM_HI - FM_LO>{});
+  if (L < FM_LO || L >= FM_HI)
+    return MixedKernel{};
+#if FM_FORM == 2
+  switch (kind) {
+  case KIND_R2C: return find<KIND_R2C>(L);
+  case KIND_C2R: return find<KIND_C2R>(L);
+  case KIND_R2C | 4: return find<(KIND_R2C | 4)>(L);
+  case KIND_C2R | 4: return find<(KIND_C2R | 4)>(L);
+  default: return MixedKernel{};
+  }
+#else
+  (void)kind;
+  return find<KIND_C2C>(L);
+#endif
 }
 
 } // namespace b200fft
