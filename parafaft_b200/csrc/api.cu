@@ -1006,6 +1006,21 @@ bool copy_covers(const H *h, const char *p, size_t n) {
   return c.active && p >= c.dst && p + n <= c.dst + c.bytes;
 }
 
+// Bytes a folded copy's source must be aligned to: the kernels load whole
+// complex points, except that R2C rows of odd length, and those of the
+// runtime-generic kernel, load single reals. (A group picks the kernel of a
+// recorded pass anew, so there a tuned plan's own choice says nothing.)
+size_t fold_unit(const H *h, const Plan &p) {
+  const bool reals = p.kind == KIND_R2C && (p.len % 2 != 0 || h->force_generic ||
+                                            (!h->recording && !p.ch.complex_units()));
+  return reals ? static_cast<size_t>(h->rsize) : h->csize();
+}
+
+bool copy_aligned(const H *h, const char *p, size_t unit) {
+  const HeldCopy &c = h->copy;
+  return reinterpret_cast<uintptr_t>(c.src + (p - c.dst)) % unit == 0;
+}
+
 int check_handle(H *h) {
   if (h == nullptr)
     return fail(B200FFT_ERR_INVALID_ARG, "b200fft: null handle");
@@ -1251,7 +1266,7 @@ int exec_real(H *h, Plan &p, int kind, void *ptr) {
   const bool dense = p.stride == 1 && p.dist == 2 * (p.len / 2 + 1);
   bool fused = false;
   if (h->copy.active) {
-    if (dense && copy_covers(h, cp, span))
+    if (dense && copy_covers(h, cp, span) && copy_aligned(h, cp, fold_unit(h, p)))
       fused = true;
     else
       B2_TRY(flush_copy(h));
@@ -1427,7 +1442,7 @@ int b200fft_exec_c2c(b200fft_handle h, int stage, int direction, void *data) {
                                          h->csize() == slab_bytes;
   bool fused = false;
   if (h->copy.active) {
-    if (dense && copy_covers(h, cp, region))
+    if (dense && copy_covers(h, cp, region) && copy_aligned(h, cp, fold_unit(h, p)))
       fused = true;
     else
       B2_TRY(flush_copy(h));
