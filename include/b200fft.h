@@ -21,7 +21,8 @@
  *     in place is folded into that transform (the transform reads the copy's
  *     source and writes the destination), which removes the identity copies
  *     that ParaFaFT's single-rank exchange_local issues between stages
- *     (parafaft_common.hpp:467-543);
+ *     (parafaft_common.hpp:467-543); a source that is not aligned to what the
+ *     transform loads is copied first;
  *   - consecutive b200fft_exec_c2c calls of one middle-axis stage on
  *     consecutive slices (the leading-dimension loop of
  *     parafaft_c2c.hpp:875-896 / parafaft_r2c.hpp:1224-1244) are merged into
@@ -221,9 +222,11 @@ int b200fft_group_stats(b200fft_group g, b200fft_stats *out);
  * power of two from 2 to 4096 (anything else returns B200FFT_ERR_UNSUPPORTED).
  * The first call on a device resolves the arrays' addresses and the first of a
  * precision fills its table on the caller's stream; make these before any
- * stream capture. The addresses are kept for the life of the process, so calls
- * after cudaDeviceReset on that device are not supported. Calls on different
- * streams may overlap. The kernel is that of an Estimate plan of the shape. */
+ * stream capture (each captured call is then one kernel; a capture that comes
+ * first captures the fill too, and its replays must not overlap other calls).
+ * The addresses are kept for the life of the process, so calls after
+ * cudaDeviceReset on that device are not supported. Calls on different streams
+ * may overlap. The kernel is that of an Estimate plan of the shape. */
 int b200fft_c2c_noalloc(int precision, int direction, int length, size_t batch,
                         ptrdiff_t stride, ptrdiff_t dist, const void *in, void *out,
                         void *cuda_stream);

@@ -23,8 +23,9 @@
 //  * the first call on a device looks up the arrays' device addresses with
 //    cudaGetSymbolAddress (once per device, with that device current), and the
 //    first call of a precision fills its table on the caller's stream; make
-//    these before any stream capture begins (a capture that comes first fills
-//    the table inside the captured work, at every replay);
+//    these before any stream capture begins: a captured call is then one kernel
+//    (and a wait for the fill where that has not finished). A capture that comes
+//    first fills the table inside the captured work, at every replay;
 //  * the addresses are kept for the life of the process: calls after
 //    cudaDeviceReset on that device are not supported (the module, and with
 //    it the arrays, may move);
@@ -63,6 +64,7 @@ struct Table {
   void *addr = nullptr;
   bool filled = false;         // the fill has finished on the device
   cudaEvent_t fill = nullptr;  // recorded after the fill until then
+  bool in_graph = false;       // a captured graph waits for that event
 };
 std::mutex g_mu;
 Table g_tables[kMaxDevices][2];
@@ -72,9 +74,18 @@ int fail(int code, const std::string &msg) {
   return code;
 }
 
+// While another stream of the process captures in global mode (the default),
+// event queries are not permitted to threads of the default capture mode and
+// would invalidate that capture. The queries below touch no captured work.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // The current device's table of one precision, ready for work that `st` runs
-// from now on.
-int device_table(bool f64, cudaStream_t st, void **out) {
+// from now on. *waits: `st` was made to wait for a fill in flight elsewhere.
+int device_table(bool f64, cudaStream_t st, bool capturing, void **out, bool *waits) {
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices)
@@ -96,32 +107,35 @@ int device_table(bool f64, cudaStream_t st, void **out) {
   *out = t.addr;
   if (t.filled)
     return B200FFT_SUCCESS;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  e = cudaStreamIsCapturing(st, &cap);
-  if (e != cudaSuccess) { // the legacy stream while another stream captures
-    cudaGetLastError();
-    cap = cudaStreamCaptureStatusActive;
-  }
-  const bool capturing = cap != cudaStreamCaptureStatusNone;
-  if (!capturing && t.fill != nullptr) {
+  const RelaxedCapture relaxed;
+  if (t.fill != nullptr) { // by an earlier call, perhaps not finished yet
     if (cudaEventQuery(t.fill) == cudaSuccess) {
       t.filled = true;
-      cudaEventDestroy(t.fill);
+      if (!t.in_graph)
+        cudaEventDestroy(t.fill);
       t.fill = nullptr;
       return B200FFT_SUCCESS;
     }
     cudaGetLastError(); // not ready yet
-    e = cudaStreamWaitEvent(st, t.fill, 0);
+    // a capture takes the wait as a node of its own, which keeps the event
+    e = cudaStreamWaitEvent(st, t.fill, capturing ? cudaEventWaitExternal : cudaEventWaitDefault);
+    t.in_graph = t.in_graph || capturing;
+    *waits = true;
   } else {
-    e = f64 ? b200fft::launch_twiddle_table(static_cast<double2 *>(t.addr), nullptr,
-                                            kNoAllocMaxLength, st)
-            : b200fft::launch_twiddle_table(nullptr, static_cast<float2 *>(t.addr),
-                                            kNoAllocMaxLength, st);
-    if (e == cudaSuccess && !capturing) {
-      e = cudaEventCreateWithFlags(&t.fill, cudaEventDisableTiming);
-      if (e == cudaSuccess)
-        e = cudaEventRecord(t.fill, st);
-    }
+    cudaEvent_t fill = nullptr;
+    if (!capturing)
+      e = cudaEventCreateWithFlags(&fill, cudaEventDisableTiming);
+    if (e == cudaSuccess)
+      e = f64 ? b200fft::launch_twiddle_table(static_cast<double2 *>(t.addr), nullptr,
+                                              kNoAllocMaxLength, st)
+              : b200fft::launch_twiddle_table(nullptr, static_cast<float2 *>(t.addr),
+                                              kNoAllocMaxLength, st);
+    if (e == cudaSuccess && !capturing)
+      e = cudaEventRecord(fill, st);
+    if (e == cudaSuccess)
+      t.fill = fill; // null in a capture: its replays fill, calls outside do too
+    else if (fill != nullptr)
+      cudaEventDestroy(fill);
   }
   if (e != cudaSuccess)
     return fail(B200FFT_ERR_CUDA,
@@ -154,8 +168,15 @@ extern "C" int b200fft_c2c_noalloc(int precision, int direction, int length, siz
                 "b200fft_c2c_noalloc: batch/stride/dist exceed the supported range");
   cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
   const bool f64 = precision == B200FFT_F64;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError(); // the legacy stream while another stream captures
+    cap = cudaStreamCaptureStatusActive;
+  }
+  const bool capturing = cap != cudaStreamCaptureStatusNone;
   void *table = nullptr;
-  const int rc = device_table(f64, st, &table);
+  bool waits = false;
+  const int rc = device_table(f64, st, capturing, &table, &waits);
   if (rc != B200FFT_SUCCESS)
     return rc;
   // level `length` of the pyramid: its table and those of the shorter lengths
@@ -169,12 +190,7 @@ extern "C" int b200fft_c2c_noalloc(int precision, int direction, int length, siz
   a.idist = a.odist = dist;
   a.istride = a.ostride = stride;
   a.islab = a.oslab = 0;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
-    cudaGetLastError(); // the legacy stream while another stream captures
-    cap = cudaStreamCaptureStatusActive;
-  }
-  a.chained = cap == cudaStreamCaptureStatusNone && // as a handle's passes
+  a.chained = !capturing && !waits && // as a handle's passes
               2 * a.total * length * (f64 ? 16 : 8) <= kChainedBytes;
   const cudaError_t e = launch_default_c2c(f64, length, dist < stride,
                                            direction == B200FFT_FORWARD, a, st);
