@@ -153,12 +153,41 @@ template <bool FWD, typename V> BF_D void dft8(V *v) {
 }
 
 // ---- 16- and 32-point butterflies from 4- and 8-point ones ---------------
-// cos and sin of 2*pi*m/n at compile time: the angle is folded by symmetry
-// into [0, pi/4] with exact integer arithmetic (in units of 1/(8n) turn), then
-// summed from the Taylor series (16 terms: far below double rounding there).
+// cos and sin of 2*pi*m/n at compile time, rounded once: the angle is folded by
+// symmetry into [0, pi/4] with exact integer arithmetic (in units of 1/(8n)
+// turn), then summed from the Taylor series in double-double numbers (Dekker's
+// two-term arithmetic; 16 terms: far below double rounding there). Summed in
+// doubles the constants were up to 2.4 units in the last place off, which was
+// most of the excess FP64 error of 7-, 25- and 49-point stages over table constants.
 struct CosSin {
   double c, s;
 };
+struct DD { // h + l, h rounded to nearest
+  double h, l;
+};
+constexpr DD dd_sum(double a, double b) { // a + b, any magnitudes
+  const double s = a + b, bb = s - a;
+  return DD{s, (a - (s - bb)) + (b - bb)};
+}
+constexpr DD dd_prod(double a, double b) {
+  const double ta = 134217729.0 * a, tb = 134217729.0 * b; // 2^27 + 1
+  const double ah = ta - (ta - a), bh = tb - (tb - b), al = a - ah, bl = b - bh;
+  const double p = a * b;
+  return DD{p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr DD dd_add(DD a, DD b) {
+  const DD s = dd_sum(a.h, b.h);
+  return dd_sum(s.h, s.l + (a.l + b.l));
+}
+constexpr DD dd_mul(DD a, DD b) {
+  const DD p = dd_prod(a.h, b.h);
+  return dd_sum(p.h, p.l + (a.h * b.l + a.l * b.h));
+}
+constexpr DD dd_div(DD a, double b) {
+  const double q = a.h / b;
+  const DD p = dd_prod(q, b);
+  return dd_sum(q, ((a.h - p.h) - p.l + a.l) / b);
+}
 constexpr CosSin ce_cossin(long long m, long long n) {
   m %= n;
   if (m < 0)
@@ -177,16 +206,17 @@ constexpr CosSin ce_cossin(long long m, long long n) {
     a = d / 4 - a;
     swap = true;
   }
-  const double x = 2.0 * 3.14159265358979323846264338327950288 * static_cast<double>(a) /
-                   static_cast<double>(d);
-  double ts = x, ss = x, tc = 1.0, sc = 1.0;
+  const DD pi2{6.283185307179586476925286766559, 2.4492935982947064e-16};
+  const DD x = dd_div(dd_mul(pi2, DD{static_cast<double>(a), 0.0}), static_cast<double>(d));
+  const DD x2 = dd_mul(x, DD{-x.h, -x.l});
+  DD ts = x, ss = x, tc{1.0, 0.0}, sc{1.0, 0.0};
   for (int k = 1; k < 16; ++k) {
-    ts *= -x * x / static_cast<double>((2 * k) * (2 * k + 1));
-    tc *= -x * x / static_cast<double>((2 * k - 1) * (2 * k));
-    ss += ts;
-    sc += tc;
+    ts = dd_div(dd_mul(ts, x2), static_cast<double>((2 * k) * (2 * k + 1)));
+    tc = dd_div(dd_mul(tc, x2), static_cast<double>((2 * k - 1) * (2 * k)));
+    ss = dd_add(ss, ts);
+    sc = dd_add(sc, tc);
   }
-  double c = swap ? ss : sc, sn = swap ? sc : ss;
+  const double c = swap ? ss.h : sc.h, sn = swap ? sc.h : ss.h;
   return CosSin{neg_c ? -c : c, neg_s ? -sn : sn};
 }
 template <int M, int N> struct TwC {

@@ -1,0 +1,75 @@
+"""Rounding errors of the compiled plans against the runtime-generic kernel of the
+same library, which loads its twiddles from the table and takes one prime (or 4,
+5, 8) at a time. The rms error against extended precision may exceed the generic
+kernel's by 8% at most: 5% that a host restatement of both arithmetics shows for
+the radix splits, 3% for the sample (2^16 points) and the order of its FMAs."""
+import numpy as np
+import pytest
+
+from helpers import cdtype, rdtype, to_dev, to_host
+from parafaft_b200 import native as nv
+
+pytestmark = pytest.mark.gpu
+
+sf = pytest.importorskip("scipy.fft")
+
+MARGIN = 1.08
+POINTS = 1 << 16
+
+
+def _rel(y, ref):
+    d = y - ref
+    return float(np.sqrt(np.sum(np.abs(d) ** 2) / np.sum(np.abs(ref) ** 2)))
+
+
+def _c2c_error(prec, n, col, flags):
+    rng = np.random.default_rng(n)
+    batch = max(2, POINTS // n)
+    shape = (n, batch) if col else (batch, n)
+    x = (rng.standard_normal(shape) + 1j * rng.standard_normal(shape)).astype(cdtype(prec))
+    h = nv.Handle(prec, 1, flags=flags)
+    h.plan_c2c(0, n, batch, *((batch, 1) if col else (1, n)))
+    d = to_dev(x)
+    h.exec_c2c(0, nv.FORWARD, d)
+    h.sync()
+    ref = sf.fft(x.astype(np.clongdouble), axis=0 if col else 1)
+    return _rel(to_host(d).astype(np.clongdouble), ref)
+
+
+def _real_errors(prec, n, flags):
+    rng = np.random.default_rng(n)
+    batch, nc = max(2, POINTS // n), n // 2 + 1
+    h = nv.Handle(prec, 0, flags=flags)
+    h.plan_r2c(n, batch, 1, 2 * nc)
+    h.plan_c2r(n, batch, 1, 2 * nc)
+    buf = np.zeros((batch, 2 * nc), rdtype(prec))
+    buf[:, :n] = rng.standard_normal((batch, n))
+    d = to_dev(buf)
+    h.exec_r2c(d)
+    h.sync()
+    fwd = _rel(to_host(d).view(cdtype(prec)).astype(np.clongdouble),
+               sf.rfft(buf[:, :n].astype(np.longdouble), axis=1))
+    X = (rng.standard_normal((batch, nc)) + 1j * rng.standard_normal((batch, nc)))
+    X[:, 0] = X[:, 0].real
+    if n % 2 == 0:
+        X[:, -1] = X[:, -1].real
+    X = X.astype(cdtype(prec))
+    d = to_dev(X.view(rdtype(prec)))
+    h.exec_c2r(d)
+    h.sync()
+    bwd = _rel(to_host(d)[:, :n].astype(np.longdouble),
+               sf.irfft(X.astype(np.clongdouble), n=n, axis=1, norm="forward"))
+    return fwd, bwd
+
+
+FP64_LENGTHS = [7, 11, 13, 14, 25, 49, 77, 91, 98, 125, 175, 196, 343, 625, 686, 875, 1225, 1372]
+
+
+@pytest.mark.parametrize("n", FP64_LENGTHS)
+def test_fp64_constants(n):
+    """Radices whose butterfly constants are formed at compile time."""
+    for col in (True, False):
+        if not col and n in (7, 11, 13):
+            continue
+        got = _c2c_error(nv.F64, n, col, 0)
+        assert got <= MARGIN * _c2c_error(nv.F64, n, col, nv.FLAG_GENERIC_ONLY), (n, col)
