@@ -9,9 +9,9 @@
 // The first stage reads global memory directly and the last stage writes it
 // directly (its write index reduces to j + r*L/R), so a transform costs one
 // HBM read and one HBM write plus (stages-1) shared-memory exchanges.
-// Twiddles come from a table exp(-2*pi*i*m/tlen) generated once per length in
-// FP64 by sincospi after exact integer reduction of m (twiddle_table_kernel),
-// then rounded to the working precision.
+// Twiddles come from a table exp(-2*pi*i*m/tlen) generated once per length after
+// exact integer reduction of m (twiddle_table_kernel), rounded to the working
+// precision.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -8,10 +8,10 @@
 namespace b200fft {
 
 // ==========================================================================
-// Twiddle tables, computed in FP64 and rounded once.
+// Twiddle tables, computed in FP64 or better and rounded once.
 // exp(-2*pi*i*m/n): 4m = q*n + r with integers q (quadrant) and r < n; the
-// angle is (pi/2)(q + r/n); the remainder is folded to [0, n/2] so sincospi
-// gets an argument in [0, 1/4] that carries no reduction error.
+// angle is (pi/2)(q + r/n); the remainder is folded to [0, n/2], so the angle
+// left is in [0, pi/4] and exact up to there (sincos_quarter).
 //
 // For a power-of-two top length M the table is a pyramid: the M-point table
 // T_M[k] = exp(-2*pi*i*k/M), then T_{M/2}, T_{M/4}, ..., T_1, with T_n at
@@ -19,6 +19,49 @@ namespace b200fft {
 // kernels index; the specialised kernels read stage twiddles w^p for
 // w = exp(-2*pi*i/n) as T_{n/p}[k], contiguous in k. Other lengths get T_M only.
 // ==========================================================================
+// cos and sin of (pi/2)(r/n), 0 <= r <= n/2: the angle, x^3/6 and x^2/2 as sums
+// of two doubles (products split by FMA), the later terms of the Taylor series
+// in doubles, where their rounding is below 2^-58 of the result. The angle
+// rounded to one double and sincospi of it were up to one unit in the last place
+// off: FP64 passes of lengths with odd prime factors had 4-5% more error, and
+// those that multiply two entries to form a third up to 10%.
+__device__ void sincos_quarter(double r, double n, double *sn, double *cs) {
+  const double qh = __ddiv_rn(r, n); // r/n = qh + ql
+  const double ql = __ddiv_rn(__fma_rn(-qh, n, r), n);
+  const double ph = 1.57079632679489661923, pl = 6.12323399573676588613e-17; // pi/2
+  double xh = __dmul_rn(ph, qh);
+  double xl = __fma_rn(ph, ql, __fma_rn(pl, qh, __fma_rn(ph, qh, -xh)));
+  const double x0 = __dadd_rn(xh, xl);
+  xl = __dsub_rn(xl, __dsub_rn(x0, xh));
+  xh = x0;
+  const double zh = __dmul_rn(xh, xh); // x^2 = zh + zl
+  const double zl = __fma_rn(2.0 * xh, xl, __fma_rn(xh, xh, -zh));
+  const double th = __dmul_rn(zh, xh); // x^3 = th + tl
+  const double tl = __fma_rn(zh, xl, __fma_rn(zl, xh, __fma_rn(zh, xh, -th)));
+  const double uh = __ddiv_rn(th, 6.0); // x^3/6 = uh + ul
+  const double ul = __ddiv_rn(__dadd_rn(__fma_rn(-uh, 6.0, th), tl), 6.0);
+  // sin x - x + x^3/6 = x^5 (1/5! - x^2/7! + ...), cos x - 1 + x^2/2 = x^4 (1/4! - ...)
+  double a = 0.0, b = 0.0;
+  const double f5[8] = {1.0 / 120, 1.0 / 5040, 1.0 / 362880, 1.0 / 39916800, 1.0 / 6227020800.0,
+                        1.0 / 1307674368000.0, 1.0 / 355687428096000.0,
+                        1.0 / 121645100408832000.0};
+  const double f4[9] = {1.0 / 24, 1.0 / 720, 1.0 / 40320, 1.0 / 3628800, 1.0 / 479001600,
+                        1.0 / 87178291200.0, 1.0 / 20922789888000.0, 1.0 / 6402373705728000.0,
+                        1.0 / 2432902008176640000.0};
+#pragma unroll
+  for (int k = 7; k >= 0; --k)
+    a = __fma_rn(-zh, a, f5[k]);
+#pragma unroll
+  for (int k = 8; k >= 0; --k)
+    b = __fma_rn(-zh, b, f4[k]);
+  a *= th * zh;
+  b *= zh * zh;
+  const double sh = __dsub_rn(xh, uh);
+  *sn = sh + (((xh - sh) - uh) + (xl - ul) + a);
+  const double hh = 0.5 * zh, ch = __dsub_rn(1.0, hh);
+  *cs = ch + (((1.0 - ch) - hh) - 0.5 * zl + b);
+}
+
 __device__ double2 twiddle_fp64(long long m, long long n) {
   const long long t = 4LL * m;
   const int q = static_cast<int>(t / n);
@@ -26,7 +69,10 @@ __device__ double2 twiddle_fp64(long long m, long long n) {
   const bool flip = 2 * r > n;
   const long long rr = flip ? (n - r) : r;
   double s, c;
-  sincospi(static_cast<double>(rr) / (2.0 * static_cast<double>(n)), &s, &c);
+  if ((n & (n - 1)) == 0) // r/n is exact, and so is sincospi but for the last rounding
+    sincospi(static_cast<double>(rr) / (2.0 * static_cast<double>(n)), &s, &c);
+  else
+    sincos_quarter(static_cast<double>(rr), static_cast<double>(n), &s, &c);
   if (flip) {
     const double tmp = s;
     s = c;

@@ -62,6 +62,24 @@ def _real_errors(prec, n, flags):
     return fwd, bwd
 
 
+@pytest.mark.parametrize("n", [17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61])
+def test_fp64_table_entries_are_rounded_once(n):
+    """The transform of an impulse at point 1 by one prime stage is the table
+    itself: within 0.6 units in the last place (half of one, and 2^-4 for the
+    series' own rounding)."""
+    h = nv.Handle(nv.F64, 1)
+    h.plan_c2c(0, n, 1, 1, n)
+    d = to_dev(np.eye(n, dtype=np.complex128)[1])
+    h.exec_c2c(0, nv.FORWARD, d)
+    h.sync()
+    w = to_host(d)
+    pi = np.longdouble("3.14159265358979323846264338327950288")
+    angle = 2 * pi * np.arange(n).astype(np.longdouble) / n
+    for got, want in ((w.real, np.cos(angle)), (w.imag, -np.sin(angle))):
+        off = np.abs(got - want)[1:] / np.spacing(np.abs(want[1:].astype(np.float64)))
+        assert off.max() < 0.6, (n, off.max())
+
+
 FP64_LENGTHS = [7, 11, 13, 14, 25, 49, 77, 91, 98, 125, 175, 196, 343, 625, 686, 875, 1225, 1372]
 
 
