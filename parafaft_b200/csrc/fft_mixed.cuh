@@ -72,11 +72,24 @@ template <int p, bool FWD, typename V> struct PrimeDft {
   }
 };
 
-// Outer factor N1 of a composite radix (the N1-point butterflies run first).
+// Outer factor N1 of a composite radix (the N1-point butterflies run first): the
+// power of 2 (of odd radices the power of 3) in it, whose cofactor then has no
+// factor in common with it; of a prime power 4, 3 or 5.
 BF_HD constexpr int mixed_outer(int R) {
-  for (int f : {4, 3, 5, 2, 7})
-    if (R % f == 0 && R > f)
-      return f;
+  for (int p = 2; p <= 3; ++p) {
+    int q = 1;
+    while (R % (p * q) == 0)
+      q *= p;
+    if (q > 1 && q < R)
+      return q;
+  }
+  return R % 4 == 0 ? 4 : R % 3 == 0 ? 3 : 5;
+}
+BF_HD constexpr int ce_gcd(int a, int b) { return b == 0 ? a : ce_gcd(b, a % b); }
+BF_HD constexpr int inverse_mod(int a, int m) { // x with x * a = 1 (mod m)
+  for (int x = 1; x < m; ++x)
+    if (a * x % m == 1)
+      return x;
   return 1;
 }
 
@@ -92,7 +105,7 @@ BF_D double2 conj_if(double2 v, unsigned flip) {
 
 template <int R, bool FWD, typename V> BF_D void dft_mixed(V *v);
 
-// CompositeDft of fft_device.cuh over the butterflies of this file.
+// CompositeDft of fft_device.cuh over the butterflies of this file (prime powers).
 template <int N1, int N2, bool FWD, typename V> struct MixedComposite {
   static constexpr int N = N1 * N2;
   template <int n2, int k1> static BF_D void twiddle_into(const V *u, V *t) {
@@ -125,41 +138,85 @@ template <int N1, int N2, bool FWD, typename V> struct MixedComposite {
   }
 };
 
+// N = N1*N2 points, N1 and N2 without a common factor (Good's prime-factor map):
+// with n = N2*n1 + N1*n2 and k = N2*(1/N2 mod N1)*k1 + N1*(1/N1 mod N2)*k2 (mod N),
+//   w_N^(n k) = w_N1^(n1 k1) w_N2^(n2 k2),
+// so no twiddles stand between the N1- and the N2-point butterflies: fewer
+// roundings (FP64 points of 2^a 3^b 5^c lengths had up to 12% more error than the
+// runtime-generic kernel's with inner twiddles at 6, 10, 12, 15, 18, 20, 24 and 30
+// points) and no constants to hold.
+template <int N1, int N2, bool FWD, typename V> struct CoprimeDft {
+  static constexpr int N = N1 * N2;
+  static constexpr int U1 = N2 * inverse_mod(N2 % N1, N1), U2 = N1 * inverse_mod(N1 % N2, N2);
+  static BF_D void run(V *v) {
+    V t[N];
+#pragma unroll
+    for (int n2 = 0; n2 < N2; ++n2) {
+      V u[N1];
+#pragma unroll
+      for (int n1 = 0; n1 < N1; ++n1)
+        u[n1] = v[(N2 * n1 + N1 * n2) % N];
+      dft_mixed<N1, FWD>(u);
+#pragma unroll
+      for (int k1 = 0; k1 < N1; ++k1)
+        t[k1 * N2 + n2] = u[k1];
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < N1; ++k1) {
+      dft_mixed<N2, FWD>(&t[k1 * N2]);
+#pragma unroll
+      for (int k2 = 0; k2 < N2; ++k2)
+        v[(U1 * k1 + U2 * k2) % N] = t[k1 * N2 + k2];
+    }
+  }
+};
+
 template <int R, bool FWD, typename V> BF_D void dft_mixed(V *v) {
   if constexpr (R <= 5 || R == 8)
     dft<R, FWD>(v);
   else if constexpr (R == 7 || R == 11 || R == 13)
     PrimeDft<R, FWD, V>::run(v);
+  else if constexpr (ce_gcd(mixed_outer(R), R / mixed_outer(R)) == 1)
+    CoprimeDft<mixed_outer(R), R / mixed_outer(R), FWD, V>::run(v);
   else
     MixedComposite<mixed_outer(R), R / mixed_outer(R), FWD, V>::run(v);
 }
 
-// v[r] *= w^r, w^r = tw[r * base] of the flat table (conjugated when CONJ):
-// w, w^2 and every w^(4a) are loaded, w^(4a+b) is w^(4a) w^b. Three powers and
-// one w^(4a) are live at a time (a chain over powers of two keeps half of all
-// powers live), no power is more than two products away from the table.
-template <int R, bool CONJ, typename V>
+// v[r] *= w^r, w^r = tw[r * base] of the flat table (conjugated when CONJ). A
+// power formed as a product carries more roundings than a loaded one, so radices
+// up to 5, in columns (whose lanes mostly share an address) up to 9, load every
+// power. Longer radices load w, w^2 and every w^(4a); the others are one product
+// each, w^(4a+1) and w^(4a+2) from the entry before, w^(4a+3) as w^(4a+4) conj(w)
+// (w^3 w^(4a) at the end of a radix). Three or four powers are live at a time (a
+// chain over powers of two keeps half of all powers live). Loading all powers of
+// radices 8 and 9 too took FP64 rows of 768 to 1008 points 30% longer, all powers
+// of any radix FP64 columns 2% longer on average and of 490, 550, 720 and 1280
+// points 13-16%.
+template <int R, bool CONJ, bool COL, typename V>
 BF_D void apply_twiddles_mixed(V *v, const V *tw, int base) {
-  if constexpr (R <= 5) {
+  if constexpr (R <= (COL ? 9 : 5)) {
 #pragma unroll
     for (int r = 1; r < R; ++r)
       v[r] = cmulw<CONJ>(v[r], ldtw(tw, r * base));
   } else {
     const V w1 = ldtw(tw, base), w2 = ldtw(tw, 2 * base);
-    const V w3 = cmulw<false>(w1, w2);
     v[1] = cmulw<CONJ>(v[1], w1);
     v[2] = cmulw<CONJ>(v[2], w2);
-    v[3] = cmulw<CONJ>(v[3], w3);
+    V wa = ldtw(tw, 4 * base);
+    v[3] = cmulw<CONJ>(v[3], cmulw<true>(wa, w1));
 #pragma unroll
     for (int a = 4; a < R; a += 4) {
-      const V wa = ldtw(tw, a * base);
       v[a] = cmulw<CONJ>(v[a], wa);
       if (a + 1 < R)
         v[a + 1] = cmulw<CONJ>(v[a + 1], cmulw<false>(wa, w1));
       if (a + 2 < R)
         v[a + 2] = cmulw<CONJ>(v[a + 2], cmulw<false>(wa, w2));
-      if (a + 3 < R)
-        v[a + 3] = cmulw<CONJ>(v[a + 3], cmulw<false>(wa, w3));
+      if (a + 4 < R) {
+        wa = ldtw(tw, (a + 4) * base);
+        v[a + 3] = cmulw<CONJ>(v[a + 3], cmulw<true>(wa, w1));
+      } else if (a + 3 < R) {
+        v[a + 3] = cmulw<CONJ>(v[a + 3], cmulw<false>(wa, cmulw<false>(w1, w2)));
+      }
     }
   }
 }
@@ -338,7 +395,7 @@ struct KM {
       // along, which keeps the code of all of them in one block)
       if (FULL || K > 1 || j < B) {
         if constexpr (s > 0)
-          apply_twiddles_mixed<R, !FWD>(&v[i * R], tw, (j % Ns) * (TSC * L / (Ns * R)));
+          apply_twiddles_mixed<R, !FWD, COL>(&v[i * R], tw, (j % Ns) * (TSC * L / (Ns * R)));
         dft_mixed<R, FWD>(&v[i * R]);
       }
     }

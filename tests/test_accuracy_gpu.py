@@ -91,3 +91,37 @@ def test_fp64_constants(n):
             continue
         got = _c2c_error(nv.F64, n, col, 0)
         assert got <= MARGIN * _c2c_error(nv.F64, n, col, nv.FLAG_GENERIC_ONLY), (n, col)
+
+
+def _good_lengths(hi):
+    out = []
+    for n in range(6, hi + 1):
+        m = n
+        for p in (2, 3, 5, 7):
+            while m % p == 0:
+                m //= p
+        if m in (1, 11, 13) and n & (n - 1):
+            out.append(n)
+    return [n for n in out if n not in (7, 11, 13)]
+
+
+@pytest.mark.parametrize("prec", [nv.F32, nv.F64])
+@pytest.mark.parametrize("part", range(4))
+def test_compiled_plans_are_as_accurate_as_the_generic_kernel(prec, part):
+    bad = []
+    for n in _good_lengths(2048)[part::4]:
+        for col in (True, False):
+            got, ref = (_c2c_error(prec, n, col, f) for f in (0, nv.FLAG_GENERIC_ONLY))
+            if not got <= MARGIN * ref:
+                bad.append((n, col, got / ref))
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("prec", [nv.F32, nv.F64])
+def test_compiled_real_rows_are_as_accurate_as_the_generic_kernel(prec):
+    bad = []
+    for n in _good_lengths(2048)[::5] + [2 * m for m in _good_lengths(2048)[2::5]]:
+        got, ref = (_real_errors(prec, n, f) for f in (0, nv.FLAG_GENERIC_ONLY))
+        if not (got[0] <= MARGIN * ref[0] and got[1] <= MARGIN * ref[1]):
+            bad.append((n, got[0] / ref[0], got[1] / ref[1]))
+    assert not bad, bad
