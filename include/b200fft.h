@@ -189,8 +189,9 @@ int b200fft_free(void *ptr);
  * recording level by level (level d: the d-th recorded pass or copy of every
  * handle): passes with a specialised kernel launch once per (precision, kind,
  * layout, direction, length), one CTA per tile of any handle's pass (a single
- * pass, and one of a mixed length above 192 points, launches its plan's own
- * kernel); the others share one persistent launch whose CTAs take (transform, tile) work items from a device queue.
+ * pass, and one of 64 MB or more on a compiled plan, launches its plan's own
+ * kernel); the others share one persistent launch whose CTAs take (transform,
+ * tile) work items from a device queue.
  * The launches of one level run side by side on several streams, so the
  * handles of a group must not share data. The recorded schedule stays valid
  * for the same buffers: group_replay runs it again, group_capture records it

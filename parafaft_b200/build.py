@@ -44,7 +44,7 @@ ENGINE_SOURCES = ["api.cu", "fg.cu", "fs_c2c_f32.cu", "fs_c2c_f64.cu",
 
 # fm_inst.cu is compiled once per precision, form (columns, rows, real rows) and
 # range of lengths; the ranges meet at kMixedCut of fm.cu.
-MIXED_RANGES = [(3, 136), (136, 351), (351, 801), (801, 2049), (4096, 4097)]
+MIXED_RANGES = [(3, 136), (136, 351), (351, 801), (801, 1201), (1201, 2049), (4096, 4097)]
 
 
 def engine_units() -> list[tuple[str, str, list[str]]]:

@@ -475,6 +475,13 @@ struct GroupStep {
 // Streams a level of a group schedule spreads its independent steps over.
 constexpr int kGroupStreams = 8;
 
+// Passes on a compiled plan that move this much launch alone, smaller ones of one
+// length share a launch: a shared launch saves 2-5 us per pass (64 grids of
+// 256x256 C2C FP32 forward+backward 90 us with a launch per row pass, 41 us
+// shared; 64 of 225x75 R2C FP64 90 and 25 us), but its CTAs read their arguments
+// from memory (3 grids of 300^3 C2C FP64 2.70 ms shared, 2.40 ms alone).
+constexpr long long kAloneBytes = 64ll << 20;
+
 struct b200fft_group_s {
   std::vector<b200fft_handle_s *> handles;
   cudaStream_t stream = nullptr;
@@ -2092,10 +2099,10 @@ int group_build(G *g) {
           !h->force_generic &&
           choose_kernel(h->prec, p.kind, p.len, p.batch, p.stride, p.dist, false, &sc) ==
               B200FFT_SUCCESS;
-      // A pass with a compiled mixed-length kernel but no grouped form of it
-      // launches on its own.
       const bool mixed = chosen && sc.mixed.one != nullptr;
-      if (mixed && sc.mixed.group == nullptr) {
+      // A large pass with a compiled kernel launches on its own (split-precision
+      // plans apart: several of them share the plain kernel's launch).
+      if (mixed && p.ch.family < 2 && pass_bytes(h, p, p.batch * op.slabs) >= kAloneBytes) {
         const long long total = p.batch * op.slabs;
         GroupStep s;
         s.type = GroupStep::SINGLE;
@@ -2105,7 +2112,7 @@ int group_build(G *g) {
         s.fwd = fwds;
         s.L = p.ch.L;
         s.h = h;
-        s.plan = p; // its own choice: split-precision and tuned plans keep theirs
+        s.plan = p; // its own choice: tuned plans keep theirs
         s.dir = op.dir;
         s.pa = pass_args(p, p.ch.complex_units(), op.in, op.out, op.tw, op.slabs, op.slab);
         s.sitems.push_back(s.pa);

@@ -11,15 +11,17 @@ namespace b200fft {
   MixedKernel fm_##p##_##f##_2(int L, int kind);                               \
   MixedKernel fm_##p##_##f##_3(int L, int kind);                               \
   MixedKernel fm_##p##_##f##_4(int L, int kind);                               \
+  MixedKernel fm_##p##_##f##_5(int L, int kind);                               \
   static MixedKernel find_##p##_##f(int L, int kind) {                         \
     return L < kMixedCut[0]   ? fm_##p##_##f##_0(L, kind)                      \
            : L < kMixedCut[1] ? fm_##p##_##f##_1(L, kind)                      \
            : L < kMixedCut[2] ? fm_##p##_##f##_2(L, kind)                      \
            : L < kMixedCut[3] ? fm_##p##_##f##_3(L, kind)                      \
-                              : fm_##p##_##f##_4(L, kind);                     \
+           : L < kMixedCut[4] ? fm_##p##_##f##_4(L, kind)                      \
+                              : fm_##p##_##f##_5(L, kind);                     \
   }
 // ranges of lengths of the compilation units (FM_LO / FM_HI in build.py)
-static constexpr int kMixedCut[4] = {136, 351, 801, 2049};
+static constexpr int kMixedCut[5] = {136, 351, 801, 1201, 2049};
 FM_DECLARE(32, 0)
 FM_DECLARE(32, 1)
 FM_DECLARE(32, 2)

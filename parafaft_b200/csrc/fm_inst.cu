@@ -69,10 +69,8 @@ cudaError_t launch_group(const PassArgs *items, const int2 *map, long long ntile
 }
 
 template <int L, int KIND, bool ODD, bool COL> constexpr MixedKernel kernel() {
-  MixedKernel k{&launch_one<L, KIND, ODD, COL>, nullptr, KM<Real, L, KIND, ODD, COL>::TB};
-  if constexpr (L <= kMixedGroupMaxL)
-    k.group = &launch_group<L, KIND, ODD, COL>;
-  return k;
+  return MixedKernel{&launch_one<L, KIND, ODD, COL>, &launch_group<L, KIND, ODD, COL>,
+                     KM<Real, L, KIND, ODD, COL>::TB};
 }
 
 // KINDX: KIND_C2C; KIND_R2C or KIND_C2R of real length 2L, or of odd length L (| 4).

@@ -102,8 +102,7 @@ cudaError_t launch_colpair_c2c_f32(int L, bool fwd, const PassArgs &a, cudaStrea
 // ignore it. `a` is in complex units on both sides, except that the real side
 // of an odd length is in reals (rows contiguous in both).
 // group: the passes of many grids, items and tile map as for the grouped
-// Family S passes (tiles of mixed_plan(...).TB transforms); lengths up to
-// kMixedGroupMaxL have it.
+// Family S passes (tiles of `tb` transforms).
 struct MixedKernel {
   cudaError_t (*one)(const PassArgs &a, unsigned flip, cudaStream_t st) = nullptr;
   cudaError_t (*group)(const PassArgs *items, const int2 *tile_map, long long ntiles,

@@ -22,10 +22,6 @@ struct MixedPlan {
 // 5, 7 and at most one 11 or 13, other than powers of two. Rows of one prime
 // stage would read a whole transform per lane, so prime rows stay generic.
 constexpr int kMixedMaxL = 2048;
-// Lengths with a grouped form too: the sides of grids small enough that many of
-// them go together (192, and R2C rows of 384); a longer axis is mostly part of a
-// pass that fills the GPU by itself.
-constexpr int kMixedGroupMaxL = 192;
 constexpr bool mixed_factors_ok(int L) {
   int m = L;
   for (int p = 2; p <= 7; ++p)
