@@ -45,15 +45,17 @@ template <bool FWD, typename V> BF_D V rot(V a) {
   return FWD ? cmake(a.y, -a.x) : cmake(-a.y, a.x);
 }
 
-// Start of a pass kernel that may be a programmatic dependent launch: let the
-// next kernel of the stream become resident as soon as every CTA of this one has
-// started, and touch no memory before the kernels in front have finished. The
-// launch and the CTAs' start-up then overlap the drain of the pass before: see
-// launch_chained for what that measured. Plain launches skip both.
+// Start of a pass kernel that may be a programmatic dependent launch: touch no
+// memory before the kernels in front have finished, then let the next kernel of
+// the stream become resident as soon as every CTA of this one has come here. The
+// launch and the start-up of the next kernel's CTAs then overlap this one: see
+// launch_chained for what that measured. The wait comes first, so that a kernel
+// behind this one, also a caller's that reads before its own wait, finds
+// everything finished that stands in front of this one. Plain launches skip both.
 BF_D void pass_begin(const PassArgs &a) {
   if (a.chained != 0) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   }
 }
 
