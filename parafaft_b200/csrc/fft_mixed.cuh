@@ -185,13 +185,15 @@ template <int R, bool FWD, typename V> BF_D void dft_mixed(V *v) {
 // v[r] *= w^r, w^r = tw[r * base] of the flat table (conjugated when CONJ). A
 // power formed as a product carries more roundings than a loaded one, so radices
 // up to 5, in columns (whose lanes mostly share an address) up to 9, load every
-// power. Longer radices load w, w^2 and every w^(4a); the others are one product
-// each, w^(4a+1) and w^(4a+2) from the entry before, w^(4a+3) as w^(4a+4) conj(w)
-// (w^3 w^(4a) at the end of a radix). Three or four powers are live at a time (a
-// chain over powers of two keeps half of all powers live). Loading all powers of
-// radices 8 and 9 too took FP64 rows of 768 to 1008 points 30% longer, all powers
-// of any radix FP64 columns 2% longer on average and of 490, 550, 720 and 1280
-// points 13-16%.
+// power. Longer radices load w, w^2 and every w^(4a) and form w^(4a+1) and
+// w^(4a+2) from the entry before. w^(4a+3) is w^(4a+4) conj(w) in FP32, one
+// product; FP64 has no registers for the entry ahead and takes w^(4a) w^3 (1125-
+// and 1701-point rows spill 108 and 316 bytes otherwise, 36 and 252 so: C2R rows
+// of 1125 reals 205 -> 219 us). Three or four powers are live at a time (a chain
+// over powers of two keeps half of all powers live). Loading all powers of radices
+// 8 and 9 too took FP64 rows of 768 to 1008 points 30% longer, all powers of any
+// radix FP64 columns 2% longer on average and of 490, 550, 720 and 1280 points
+// 13-16%.
 template <int R, bool CONJ, bool COL, typename V>
 BF_D void apply_twiddles_mixed(V *v, const V *tw, int base) {
   if constexpr (R <= (COL ? 9 : 5)) {
@@ -199,11 +201,16 @@ BF_D void apply_twiddles_mixed(V *v, const V *tw, int base) {
     for (int r = 1; r < R; ++r)
       v[r] = cmulw<CONJ>(v[r], ldtw(tw, r * base));
   } else {
+    constexpr bool AHEAD = sizeof(V) == 8;
     const V w1 = ldtw(tw, base), w2 = ldtw(tw, 2 * base);
+    V wa = ldtw(tw, 4 * base), w3;
+    if constexpr (AHEAD)
+      w3 = cmulw<true>(wa, w1);
+    else
+      w3 = cmulw<false>(w1, w2);
     v[1] = cmulw<CONJ>(v[1], w1);
     v[2] = cmulw<CONJ>(v[2], w2);
-    V wa = ldtw(tw, 4 * base);
-    v[3] = cmulw<CONJ>(v[3], cmulw<true>(wa, w1));
+    v[3] = cmulw<CONJ>(v[3], w3);
 #pragma unroll
     for (int a = 4; a < R; a += 4) {
       v[a] = cmulw<CONJ>(v[a], wa);
@@ -211,12 +218,12 @@ BF_D void apply_twiddles_mixed(V *v, const V *tw, int base) {
         v[a + 1] = cmulw<CONJ>(v[a + 1], cmulw<false>(wa, w1));
       if (a + 2 < R)
         v[a + 2] = cmulw<CONJ>(v[a + 2], cmulw<false>(wa, w2));
-      if (a + 4 < R) {
+      const V here = wa;
+      if (a + 4 < R)
         wa = ldtw(tw, (a + 4) * base);
-        v[a + 3] = cmulw<CONJ>(v[a + 3], cmulw<true>(wa, w1));
-      } else if (a + 3 < R) {
-        v[a + 3] = cmulw<CONJ>(v[a + 3], cmulw<false>(wa, cmulw<false>(w1, w2)));
-      }
+      if (a + 3 < R)
+        v[a + 3] = cmulw<CONJ>(v[a + 3], AHEAD && a + 4 < R ? cmulw<true>(wa, w1)
+                                                            : cmulw<false>(here, w3));
     }
   }
 }
