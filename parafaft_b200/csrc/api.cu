@@ -258,7 +258,7 @@ int choose_kernel(int prec, int kind, int len, long long batch, long long stride
       (kind == KIND_C2C || (!odd && stride == 1 && dist % 2 == 0 && L <= 2048));
   if (static_ok) {
     const int tile = default_variant(csize, L, ch.col, stride);
-    const bool compiled_row = !ch.col && mixed_pow2_row(L, csize, kind != KIND_C2C);
+    const bool compiled_row = !ch.col && mixed_pow2_row(L, csize, kind);
     int var = compiled_row ? kVariantCompiled : tile;
     if (const char *v = std::getenv("B200FFT_VARIANT")) {
       char *end = nullptr;
@@ -969,7 +969,7 @@ namespace b200fft {
 cudaError_t launch_default_c2c(bool f64, int L, bool col, bool fwd, const PassArgs &a,
                                cudaStream_t st) {
   const int csz = f64 ? 16 : 8;
-  if (!col && mixed_pow2_row(L, csz, false))
+  if (!col && mixed_pow2_row(L, csz, KIND_C2C))
     return mixed_kernel(f64, KIND_C2C, false, false, L).one(a, fwd ? 0u : 0x80000000u, st);
   int var = default_variant(csz, L, col, a.istride);
   if (col) {

@@ -34,7 +34,7 @@ MixedKernel mixed_kernel(bool f64, int kind, bool odd, bool col, int L) {
   if (kind != KIND_C2C && col)
     return MixedKernel{};
   if (!mixed_length_ok(L, col) &&
-      (col || !mixed_pow2_row(L, f64 ? 16 : 8, kind != KIND_C2C)))
+      (col || !mixed_pow2_row(L, f64 ? 16 : 8, kind)))
     return MixedKernel{};
   if (kind == KIND_C2C)
     return f64 ? (col ? find_64_0(L, kind) : find_64_1(L, kind))

@@ -79,10 +79,10 @@ template <int L, int KINDX> constexpr MixedKernel entry() {
   if constexpr (mixed_length_ok(L, true))
     return kernel<L, KIND_C2C, false, true>();
 #elif FM_FORM == 1
-  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), false))
+  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), KIND_C2C))
     return kernel<L, KIND_C2C, false, false>();
 #else
-  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), true)) {
+  if constexpr (mixed_length_ok(L, false) || mixed_pow2_row(L, 2 * sizeof(Real), KINDX & 3)) {
     if constexpr ((KINDX & 4) == 0)
       return kernel<L, KINDX, false, false>();
     else if constexpr (L % 2 == 1)

@@ -45,14 +45,20 @@ constexpr bool mixed_length_ok(int L, bool col) {
 //   C2C FP64: 8 3.5 -> 5.6, 16 5.5 -> 6.5, 128 5.7 -> 6.2, 256 6.3 -> 6.4,
 //     2048 5.0 -> 5.2 (32, 64, 512, 1024 and 4096 stay: 6.5, 6.4, 6.2 -> 5.7, 5.1,
 //     5.5 -> 4.8);
+//   R2C FP32 of 2 x 8 3.4 -> 5.5, 2 x 16 4.1 -> 4.5, 2 x 64 5.6 -> 5.7, 2 x 128 5.4 ->
+//     5.8 (2 x 256 stays; 2 x 1024 5.5 -> 5.4 and 2 x 2048 4.2 -> 4.1 stay);
+//   R2C FP64 of 2 x 8 4.7 -> 5.3, 2 x 16 4.7 -> 5.7, 2 x 64 5.8 -> 6.3, 2 x 128 5.2 ->
+//     5.6, 2 x 256 5.3 -> 5.5, 2 x 1024 3.9 -> 4.5, 2 x 2048 3.8 -> 4.3 (2 x 512 stays);
 //   C2R FP32 of 2 x 16 3.5 -> 4.4, 2 x 128 5.4 -> 5.6, 2 x 1024 4.3 -> 5.1,
 //     2 x 2048 2.0 -> 3.8 (2 x 256 5.8 -> 5.6 stays);
 //   C2R FP64 of 2 x 16 4.5 -> 5.7, 2 x 64 5.7 -> 5.9, 2 x 1024 2.8 -> 4.0,
 //     2 x 2048 2.8 -> 4.1 (2 x 512 4.8 -> 4.3 stays).
-constexpr bool mixed_pow2_row(int L, int es, bool real) {
+constexpr bool mixed_pow2_row(int L, int es, int kind) {
   if (L < 8 || !is_pow2(L))
     return false;
-  if (real)
+  if (kind == KIND_R2C && es == 8 && L >= 1024)
+    return false;
+  if (kind != KIND_C2C)
     return L <= 2048 && !(es == 8 && L == 256) && !(es == 16 && L == 512);
   return es == 8 ? L <= 4096 && L != 1024
                  : L <= 2048 && L != 32 && L != 64 && L != 512 && L != 1024;
