@@ -125,3 +125,32 @@ def test_compiled_real_rows_are_as_accurate_as_the_generic_kernel(prec):
         if not (got[0] <= MARGIN * ref[0] and got[1] <= MARGIN * ref[1]):
             bad.append((n, got[0] / ref[0], got[1] / ref[1]))
     assert not bad, bad
+
+
+@pytest.mark.parametrize("prec", [nv.F32, nv.F64])
+@pytest.mark.parametrize("n", [16, 32, 64, 128, 256, 512, 1024, 2048])
+def test_small_column_tiles_are_as_accurate_as_the_full_tile(monkeypatch, prec, n):
+    """Few columns run on smaller tiles with shorter stages, through handles and
+    through the entry point without one. The margin: 1% of the radix split (host
+    restatement), 3% for the sample and the order of FMAs."""
+    import torch
+    rng = np.random.default_rng(n)
+    b = max(8, (1 << 16) // n)
+    x = (rng.standard_normal((n, b)) + 1j * rng.standard_normal((n, b))).astype(cdtype(prec))
+    ref = sf.fft(x.astype(np.clongdouble), axis=0)
+    small = to_dev(np.zeros_like(x))
+    src = to_dev(x)
+    torch.cuda.synchronize()
+    nv.c2c_noalloc(prec, nv.FORWARD, n, b, b, 1, src, small)
+    monkeypatch.setenv("B200FFT_VARIANT", "0")
+    # enough columns for full tiles: the batch repeated side by side, beyond two
+    # tiles per SM
+    reps = -(-2 * 148 * 8192 // (n * b)) + 1
+    h = nv.Handle(prec, 1)
+    h.plan_c2c(0, n, b * reps, b * reps, 1)
+    full = to_dev(np.tile(x, (1, reps)))
+    h.exec_c2c(0, nv.FORWARD, full)
+    h.sync()
+    got = _rel(to_host(small).astype(np.clongdouble), ref)
+    want = _rel(to_host(full)[:, :b].astype(np.clongdouble), ref)
+    assert got <= 1.04 * want, got / want
