@@ -104,3 +104,43 @@ def test_misaligned_sources_give_the_oracle_values(prec, n, offset):
     h.sync()
     ref = O.c2c_batch(z.astype(np.complex128), n, batch, 1, n, -1)
     assert O.rel_l2(to_host(dst), ref) < tol(prec)
+
+
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("n,offset,extra,folds", [
+    (100, 0, 0, True), (100, 1, 0, True), (100, 0, 1, True), (100, 0, 2, True),
+    (350, 1, 1, True), (75, 1, 1, True), (120, 0, 1, False), (128, 1, 0, False),
+    (128, 0, 2, True)])
+def test_pads_fold_real_aligned_sources(prec, n, offset, extra, folds):
+    """A pad whose source is aligned to or pitched by single reals folds into the
+    R2C pass of every length without a specialised kernel."""
+    es, pitch = (8 if prec == nv.F64 else 4), 2 * (n // 2 + 1)
+    h = _handle(prec, nv.FLAG_RECORD_ONLY)
+    run, _ = _plan(h, "r2c", n, 5)
+    h.memcpy2d(BASE_DST, pitch * es, BASE_SRC + offset * es, (n + extra) * es, n * es, 5)
+    run(BASE_DST)
+    h.flush()
+    st = h.stats()
+    assert (st["fused_copies"], st["copies_issued"]) == (int(folds), int(not folds)), st
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec", PRECS)
+@pytest.mark.parametrize("n", [36, 100, 350, 1000, 75, 120])
+@pytest.mark.parametrize("offset,extra", [(0, 0), (1, 0), (0, 1), (1, 3)])
+def test_pads_give_the_oracle_values(prec, n, offset, extra):
+    batch, nc = 21, n // 2 + 1
+    rows = O.normal_real((batch, n + extra), n).astype(rdtype(prec))
+    src = to_dev(np.concatenate([np.zeros(offset, rdtype(prec)), rows.reshape(-1)]))
+    dst = to_dev(np.zeros(batch * 2 * nc, rdtype(prec)))
+    h = _handle(prec)
+    run, _ = _plan(h, "r2c", n, batch)
+    es = rows.itemsize
+    for _ in range(2):  # the plan keeps its kernel for aligned rows
+        h.memcpy2d(dst, 2 * nc * es, src.data_ptr() + offset * es, (n + extra) * es, n * es,
+                   batch)
+        run(dst)
+        h.sync()
+        X = to_host(dst).view(cdtype(prec)).reshape(batch, nc)
+        ref = np.stack([O.r2c_nd(r) for r in rows[:, :n].astype(np.float64)])
+        assert O.rel_l2(X, ref) < tol(prec)
