@@ -30,6 +30,12 @@
  * Held-back work is issued by the next call on the handle that does not extend
  * it and by b200fft_sync()/b200fft_flush(). Create the handle with
  * B200FFT_FLAG_NO_DEFER to issue every call immediately.
+ *
+ * Passes of up to 128 MB of traffic may launch with the programmatic stream
+ * serialization attribute: they wait for the kernel in front of them on the
+ * device, and let a kernel behind them that has the attribute start after that.
+ * A kernel of the caller's in front of one that was itself launched with the
+ * attribute has to wait (cudaGridDependencySynchronize) before it ends.
  */
 #ifndef B200FFT_H
 #define B200FFT_H
@@ -164,7 +170,9 @@ int b200fft_flush(b200fft_handle h);
  * parafaft_r2c.hpp:1174-1203); B200Backend forwards it here. bytes = 0 means
  * "large enough for every plan's layout". */
 int b200fft_set_work_buffer(b200fft_handle h, void *work, size_t bytes);
-/* The kernel a plan uses (kind 0 c2c with `stage`, 1 r2c, 2 c2r). */
+/* The kernel a plan uses (kind 0 c2c with `stage`, 1 r2c, 2 c2r). Where the text
+ * has "compiled=", that compiled plan runs; the fields before it are the tile the
+ * length would have without one. */
 int b200fft_plan_describe(b200fft_handle h, int kind, int stage, char *buf,
                           size_t buflen);
 /* Plan cache, the analogue of FFTW wisdom (fft_backend_fftw.hpp:666-694):

@@ -437,8 +437,8 @@ struct b200fft_handle_s {
 namespace {
 
 struct GroupStep {
-  // SINGLE: a level's only pass of its (length, layout, kind, direction): it
-  // runs the plan's own kernel choice (tile variant, TMA or tensor-core form)
+  // SINGLE: a level's only pass of its (length, layout, kind, direction), or a
+  // large one on a compiled plan: it runs the plan's own kernel choice (tile variant, TMA or tensor-core form)
   // on the group's stream rather than the grouped kernel's default tile.
   enum { PASSES = 0, COPY = 1, COPY2D = 2, STATIC = 3, SINGLE = 4 };
   int type = PASSES;

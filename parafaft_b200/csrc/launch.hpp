@@ -11,7 +11,7 @@ namespace b200fft {
 // CTAs may become resident while the kernel before it on the stream drains; they
 // wait for it on the device (pass_begin), so the order of memory accesses is that
 // of a plain launch. Passes that move up to kChainedBytes (what the L2 holds)
-// launch so: forward+backward of 512 columns of 128 FP32 points 13.5 -> 12.1 us,
+// launch so: forward+backward of 512 columns of 128 FP32 points 13.5 -> 12.6 us,
 // 64^3 FP32 graphs 10.3 -> 8.2 us per transform, 128^3 FP32 22.3 -> 20.5. Above
 // that the gap between passes no longer counts, and the waiting CTAs of the next
 // pass cost more than it: 256^3 R2C FP64 321 -> 328 us.
