@@ -29,7 +29,10 @@ inline cudaError_t launch_chained(bool chained, void (*kern)(KArgs...), unsigned
   at.val.programmaticStreamSerializationAllowed = 1;
   c.attrs = &at;
   c.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&c, kern, static_cast<KArgs>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&c, kern, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess)
+    cudaGetLastError(); // returned here, and not again by the next launch that asks
+  return e;
 }
 
 // Family S: specialised kernels for power-of-two stage lengths L.

@@ -137,9 +137,11 @@ int device_table(bool f64, cudaStream_t st, bool capturing, void **out, bool *wa
     else if (fill != nullptr)
       cudaEventDestroy(fill);
   }
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError(); // reported here
     return fail(B200FFT_ERR_CUDA,
                 std::string("b200fft_c2c_noalloc: twiddle table: ") + cudaGetErrorString(e));
+  }
   return B200FFT_SUCCESS;
 }
 

@@ -3,6 +3,8 @@ launched with the programmatic attribute that reads before its wait finds what a
 kernel two places in front of it wrote."""
 import ctypes as C
 import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -70,3 +72,76 @@ def test_early_reads_behind_chained_passes(tmp_path):
         assert np.array_equal(to_host(out), want), i
     h.set_stream(None)
     cu.cuModuleUnload(mod)
+
+
+LAUNCH_ERROR = r"""
+import ctypes as C, sys
+sys.path[:0] = [%r, %r]
+import numpy as np, torch
+from helpers import to_dev, to_host
+from oracle import oracle as O
+from parafaft_b200 import native as nv
+cu = C.CDLL("libcuda.so.1")
+n, b = 64, 40
+x = O.normal_complex(n * b, 1).astype(np.complex64)
+d = to_dev(x)
+out = torch.empty_like(d)
+for _ in range(2):
+    nv.c2c_noalloc(nv.F32, nv.FORWARD, n, b, b, 1, d, out)
+    torch.cuda.synchronize()
+s = C.c_void_p()  # a stream that the default stream would have to wait for
+assert cu.cuStreamCreate(C.byref(s), 0) == 0
+assert cu.cuStreamBeginCapture_v2(s, 2) == 0
+try:
+    nv.c2c_noalloc(nv.F32, nv.FORWARD, n, b, b, 1, d, out)
+    raise SystemExit("the launch was accepted")
+except nv.B200FFTError as e:
+    assert "transform kernel" in str(e), e
+g = C.c_void_p()
+cu.cuStreamEndCapture(s, C.byref(g))
+h = nv.Handle(nv.F32, 1)
+h.plan_c2c(0, 17, 8, 1, 17)  # a table and a launch that ask for the last error
+y = O.normal_complex(17 * 8, 2).astype(np.complex64)
+e = to_dev(y)
+h.exec_c2c(0, nv.FORWARD, e)
+h.sync()
+assert O.rel_l2(to_host(e), O.c2c_batch(y.astype(np.complex128), 17, 8, 1, 17, -1)) < 2e-6
+"""
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """A call on the default stream while a stream it synchronises with captures is
+    refused; the next call does not report that error again."""
+    root = Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", LAUNCH_ERROR % (str(root), str(root / "tests"))],
+                       capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("prec", [nv.F32, nv.F64])
+def test_default_stream_chains_wait_for_blocking_streams(prec):
+    """Chained calls on the default stream with passes of a handle's own (blocking)
+    stream in between: the same bits as waiting after every call."""
+    import torch
+    n, b = 512, 6000
+    x = O.normal_complex(n * b, 3).astype(np.complex64 if prec == nv.F32 else np.complex128)
+    a = to_dev(x)
+    y, z = torch.empty_like(a), torch.empty_like(a)
+    h = nv.Handle(prec, 1)
+    h.plan_c2c(0, n, b, b, 1)
+
+    def run(wait):
+        step = torch.cuda.synchronize if wait else (lambda: None)
+        for _ in range(4):
+            nv.c2c_noalloc(prec, nv.FORWARD, n, b, 1, n, a, y); step()
+            h.exec_c2c(0, nv.FORWARD, y); step()
+            nv.c2c_noalloc(prec, nv.BACKWARD, n, b, 1, n, y, z); step()
+        torch.cuda.synchronize()
+        return to_host(z)
+
+    torch.cuda.synchronize()
+    want = run(True)
+    for _ in range(3):
+        z.zero_()
+        torch.cuda.synchronize()
+        assert np.array_equal(run(False), want)
