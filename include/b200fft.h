@@ -235,7 +235,8 @@ int b200fft_group_stats(b200fft_group g, b200fft_stats *out);
  * first captures the fill too, and its replays must not overlap other calls).
  * The addresses are kept for the life of the process, so calls after
  * cudaDeviceReset on that device are not supported. Calls on different streams
- * may overlap. The kernel is that of an Estimate plan of the shape. */
+ * may overlap. The kernel is that of an Estimate plan of the shape (few FP64
+ * columns of 128, 256 or 1024 points: the full tile). */
 int b200fft_c2c_noalloc(int precision, int direction, int length, size_t batch,
                         ptrdiff_t stride, ptrdiff_t dist, const void *in, void *out,
                         void *cuda_stream);

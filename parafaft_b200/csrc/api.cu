@@ -892,6 +892,13 @@ int column_tile(int csz, int L, int var, long long total, int sms) {
   return 2;
 }
 
+// Radix stages of a specialised column tile.
+int column_stages(int csz, int L, int var) {
+  const CfgS c = cfg_static(csz, L, true, var);
+  int r[24] = {}, rest = 1;
+  return static_schedule(L, radix_cap(csz, L, c.TB, c.NT), 0, r, rest);
+}
+
 int column_tile_for(const H *h, const Plan &p, long long total) {
   if (h->plan_flag != B200FFT_PLAN_ESTIMATE || !p.ch.col || !is_pow2(p.ch.L))
     return p.ch.variant;
@@ -975,7 +982,11 @@ cudaError_t launch_default_c2c(bool f64, int L, bool col, bool fwd, const PassAr
   if (col) {
     int dev = -1;
     cudaGetDevice(&dev);
-    var = column_tile(csz, L, var, a.total, device_sms(dev));
+    const int small = column_tile(csz, L, var, a.total, device_sms(dev));
+    // FP64: not a smaller tile with more stages, whose error is 2-3% above the full
+    // tile's (128, 256 and 1024 points; FP32 ones load their twiddles instead)
+    if (!f64 || column_stages(csz, L, small) <= column_stages(csz, L, var))
+      var = small;
     if (pair_by_default(f64, L, var, a))
       return launch_colpair_c2c_f32(L, fwd, a, st);
   }

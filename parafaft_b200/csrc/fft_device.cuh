@@ -448,13 +448,15 @@ struct KS {
   static constexpr bool CHAINS = sizeof(V) == 8;
   static_assert(NT % TB == 0, "TB must divide NT");
   static_assert(S.rest == 1, "length not factorable");
-  // Half and quarter column tiles (passes too small to fill the GPU) whose stages
-  // are more and shorter than the full tile's have more twiddles; they load every
-  // one, which keeps their error at the full tile's (32 FP32 points 8% above it
-  // with formed powers, 128 points 3%). Their lanes mostly share an address.
+  // FP32 half and quarter column tiles (passes too small to fill the GPU) of up to
+  // 128 points whose stages are more and shorter than the full tile's have more
+  // twiddles; they load every one, which keeps their error at the full tile's (32
+  // points 8% above it with formed powers, 128 points 3%). Their lanes mostly share
+  // an address. Longer ones are within 2% of it without, and the loads cost them 7-10%
+  // (16 MB of 512 points 8.7 -> 9.6 us); so it is in FP64 (128 points 8.9 -> 10.4).
   static constexpr bool load_all() {
     constexpr int ES = int(sizeof(V));
-    if (!COL || KIND != KIND_C2C || !is_pow2(L) || TB * L >= (ES == 8 ? 8192 : 4096))
+    if (!COL || KIND != KIND_C2C || ES != 8 || !is_pow2(L) || L > 128 || TB * L >= 8192)
       return false;
     constexpr CfgS full = cfg_static(ES, L, true, 0);
     constexpr SchedS<L, radix_cap(ES, L, full.TB, full.NT), 0> F{};

@@ -114,7 +114,8 @@ struct MixedKernel {
 };
 MixedKernel mixed_kernel(bool f64, int kind, bool odd, bool col, int L);
 
-// The kernel of an Estimate plan of a power-of-two C2C pass (api.cu).
+// The kernel of an Estimate plan of a power-of-two C2C pass (api.cu; few FP64
+// columns: the full tile).
 cudaError_t launch_default_c2c(bool f64, int L, bool col, bool fwd, const PassArgs &a,
                                cudaStream_t st);
 

@@ -29,7 +29,8 @@
 //  * the addresses are kept for the life of the process: calls after
 //    cudaDeviceReset on that device are not supported (the module, and with
 //    it the arrays, may move);
-//  * the transform runs the kernel an Estimate plan of the same shape takes;
+//  * the transform runs the kernel an Estimate plan of the same shape takes (few
+//    FP64 columns of 128, 256 or 1024 points the full tile);
 //  * calls on different streams need no ordering among themselves: until the
 //    fill has finished, calls on other streams wait for it (on the device).
 #include <cuda_runtime.h>
